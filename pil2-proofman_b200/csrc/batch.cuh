@@ -6,7 +6,7 @@
 // phase for every instance of the batch:
 //   * grouped transpose, one launch per NTT window index (instances aligned on their last
 //     inverse window and on their first forward window), one launch per tree level index;
-//   * the leaf sponge is a persistent kernel: one resident CTA per SM slot pulls 128-row
+//   * the leaf sponge is a persistent kernel: the four thread groups of one CTA per SM pull 128-row
 //     blocks of any instance from a device work counter until all rows are hashed, so
 //     instances of uneven size share the machine without tail effects;
 // and the whole sequence is captured once in a CUDA graph and replayed (BatchPlan).
@@ -160,36 +160,45 @@ inline cudaError_t set_grouped_fixed_attrs()
     return cudaSuccess;
 }
 
-// Persistent leaf sponge: CTAs claim 128-row blocks from *counter until `total` is reached.
+// Persistent leaf sponge: the groups of every CTA claim 128-row blocks from *counter until `total` is reached.
 template <int W, int FAM>
-__global__ void __launch_bounds__(merkle::TPB, merkle::Family<FAM>::MIN_CTAS)
+__global__ void __launch_bounds__(tch::THREADS, 1)
     leaf_persistent(const LeafEntry *e, int n, uint64_t total, unsigned long long *counter)
 {
-    __shared__ uint64_t sm[merkle::Family<FAM>::SMEM_AREAS * W * merkle::TPB];
-    __shared__ uint64_t claim;
-    __shared__ LeafEntry L;  // the claimed block's instance, staged for the CTA
+    extern __shared__ __align__(128) uint8_t tc_sm[];
+    __shared__ tch::Shared sh;
+    __shared__ uint64_t claim[tch::GROUPS];
+    __shared__ LeafEntry entry[tch::GROUPS];  // the claimed block's instance, staged for the group
+    tch::Group<W, FAM> G;
+    G.setup(tc_sm, sh);
     for (;;) {
-        if (threadIdx.x == 0) {
-            claim = atomicAdd(counter, 1ull);
-            if (claim < total) L = e[find_entry(e, n, claim)];
+        if (G.issuer) {
+            const uint64_t b = atomicAdd(counter, 1ull);
+            claim[G.id] = b;
+            if (b < total) entry[G.id] = e[find_entry(e, n, b)];
         }
-        __syncthreads();
-        const uint64_t b = claim;
-        if (b >= total) return;
-        const uint64_t row = (b - L.begin) * merkle::TPB + threadIdx.x;
-        if (row < L.nrows) merkle::leaf_row<W, FAM>(sm + threadIdx.x, L.digests, L.src, 1, L.nrows, L.ncols, row);
-        __syncthreads();
+        G.sync();
+        const uint64_t b = claim[G.id];
+        if (b >= total) break;
+        const LeafEntry &L = entry[G.id];
+        tch::leaf_tile(G, L.digests, L.src, 1, L.nrows, L.ncols, L.nrows, b - L.begin, false);
+        G.sync();
     }
+    G.finish(sh);
 }
 
 template <int W, int FAM>
-__global__ void __launch_bounds__(merkle::TPB, merkle::Family<FAM>::MIN_CTAS) node_grouped(const NodeEntry *e, int n)
+__global__ void __launch_bounds__(tch::THREADS, 1) node_grouped(const NodeEntry *e, int n, uint64_t total)
 {
-    __shared__ uint64_t sm[merkle::Family<FAM>::SMEM_AREAS * W * merkle::TPB];
-    const int i = find_entry(e, n, blockIdx.x);
-    const NodeEntry E = e[i];
-    const uint64_t idx = (blockIdx.x - E.begin) * merkle::TPB + threadIdx.x;
-    if (idx < E.parents) merkle::node_one<W, FAM>(sm + threadIdx.x, E.level, E.pending, E.pad, E.parents, E.out, idx);
+    extern __shared__ __align__(128) uint8_t tc_sm[];
+    __shared__ tch::Shared sh;
+    tch::Group<W, FAM> G;
+    G.setup(tc_sm, sh);
+    for (uint64_t b = blockIdx.x + (uint64_t)gridDim.x * G.id; b < total; b += (uint64_t)gridDim.x * tch::GROUPS) {
+        const NodeEntry &E = e[find_entry(e, n, b)];
+        tch::node_tile(G, E.level, E.pending, E.pad, E.parents, E.out, b - E.begin);
+    }
+    G.finish(sh);
 }
 
 __global__ void gather_roots(const uint64_t *const *tree_ends, int n, uint64_t *roots)
@@ -222,6 +231,27 @@ struct Launch {
     uint64_t ncols = 0; // kind 6
     int inst = -1;      // kind 7
 };
+
+// shared memory limit of the grouped hashing kernels
+template <int W, int FAM>
+inline cudaError_t set_hash_attrs()
+{
+    const cudaError_t e = cudaFuncSetAttribute(leaf_persistent<W, FAM>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               tch::Smem<W>::BYTES);
+    if (e != cudaSuccess) return e;
+    return cudaFuncSetAttribute(node_grouped<W, FAM>, cudaFuncAttributeMaxDynamicSharedMemorySize, tch::Smem<W>::BYTES);
+}
+
+inline cudaError_t set_grouped_hash_attrs()
+{
+    cudaError_t e = set_hash_attrs<8, 1>();
+    if (e == cudaSuccess) e = set_hash_attrs<8, 2>();
+    if (e == cudaSuccess) e = set_hash_attrs<12, 1>();
+    if (e == cudaSuccess) e = set_hash_attrs<12, 2>();
+    if (e == cudaSuccess) e = set_hash_attrs<16, 1>();
+    if (e == cudaSuccess) e = set_hash_attrs<16, 2>();
+    return e;
+}
 
 class Plan {
   public:
@@ -426,7 +456,7 @@ class Plan {
                 if (x.arity != ar) continue;
                 const uint64_t NExt = 1ull << x.nBitsExt;
                 LeafEntry e{x.lde, x.tree, x.nCols, NExt, b};
-                b += (NExt + merkle::TPB - 1) / merkle::TPB;
+                b += (NExt + 127) / 128;
                 le.push_back(e);
             }
             if (le.empty()) continue;
@@ -450,7 +480,7 @@ class Plan {
                     if (pending <= 1) continue;
                     const uint64_t pad = (ar - pending % ar) % ar, parents = (pending + ar - 1) / ar;
                     NodeEntry e{x.tree + base, x.tree + base + (pending + pad) * 4, pending, pad, parents, nb};
-                    nb += (parents + merkle::TPB - 1) / merkle::TPB;
+                    nb += (parents + 127) / 128;
                     ne.push_back(e);
                 }
                 if (ne.empty()) break;
@@ -466,8 +496,7 @@ class Plan {
         roots_off = push(zeros);
         std::vector<unsigned long long> ctr(n_counters ? n_counters : 1, 0ull);
         counters_off = push(ctr);
-        leaf_ctas = sm_count * merkle::Family<2>::MIN_CTAS;
-        if (family == 1) leaf_ctas = sm_count * merkle::Family<1>::MIN_CTAS;
+        leaf_ctas = sm_count;
         return true;
     }
 
@@ -513,26 +542,27 @@ class Plan {
                 const unsigned ctas = (unsigned)std::min<uint64_t>(L.blocks, (uint64_t)leaf_ctas);
                 const LeafEntry *le = (const LeafEntry *)ent;
                 if (family == 1) {
-                    if (L.width == 8) leaf_persistent<8, 1><<<ctas, merkle::TPB, 0, s>>>(le, L.n, L.blocks, ctr + L.smem);
-                    if (L.width == 12) leaf_persistent<12, 1><<<ctas, merkle::TPB, 0, s>>>(le, L.n, L.blocks, ctr + L.smem);
-                    if (L.width == 16) leaf_persistent<16, 1><<<ctas, merkle::TPB, 0, s>>>(le, L.n, L.blocks, ctr + L.smem);
+                    if (L.width == 8) leaf_persistent<8, 1><<<ctas, tch::THREADS, tch::Smem<8>::BYTES, s>>>(le, L.n, L.blocks, ctr + L.smem);
+                    if (L.width == 12) leaf_persistent<12, 1><<<ctas, tch::THREADS, tch::Smem<12>::BYTES, s>>>(le, L.n, L.blocks, ctr + L.smem);
+                    if (L.width == 16) leaf_persistent<16, 1><<<ctas, tch::THREADS, tch::Smem<16>::BYTES, s>>>(le, L.n, L.blocks, ctr + L.smem);
                 } else {
-                    if (L.width == 8) leaf_persistent<8, 2><<<ctas, merkle::TPB, 0, s>>>(le, L.n, L.blocks, ctr + L.smem);
-                    if (L.width == 12) leaf_persistent<12, 2><<<ctas, merkle::TPB, 0, s>>>(le, L.n, L.blocks, ctr + L.smem);
-                    if (L.width == 16) leaf_persistent<16, 2><<<ctas, merkle::TPB, 0, s>>>(le, L.n, L.blocks, ctr + L.smem);
+                    if (L.width == 8) leaf_persistent<8, 2><<<ctas, tch::THREADS, tch::Smem<8>::BYTES, s>>>(le, L.n, L.blocks, ctr + L.smem);
+                    if (L.width == 12) leaf_persistent<12, 2><<<ctas, tch::THREADS, tch::Smem<12>::BYTES, s>>>(le, L.n, L.blocks, ctr + L.smem);
+                    if (L.width == 16) leaf_persistent<16, 2><<<ctas, tch::THREADS, tch::Smem<16>::BYTES, s>>>(le, L.n, L.blocks, ctr + L.smem);
                 }
                 break;
             }
             case 3: {
+                const unsigned ctas = (unsigned)std::min<uint64_t>(L.blocks, (uint64_t)leaf_ctas);
                 const NodeEntry *ne = (const NodeEntry *)ent;
                 if (family == 1) {
-                    if (L.width == 8) node_grouped<8, 1><<<(unsigned)L.blocks, merkle::TPB, 0, s>>>(ne, L.n);
-                    if (L.width == 12) node_grouped<12, 1><<<(unsigned)L.blocks, merkle::TPB, 0, s>>>(ne, L.n);
-                    if (L.width == 16) node_grouped<16, 1><<<(unsigned)L.blocks, merkle::TPB, 0, s>>>(ne, L.n);
+                    if (L.width == 8) node_grouped<8, 1><<<ctas, tch::THREADS, tch::Smem<8>::BYTES, s>>>(ne, L.n, L.blocks);
+                    if (L.width == 12) node_grouped<12, 1><<<ctas, tch::THREADS, tch::Smem<12>::BYTES, s>>>(ne, L.n, L.blocks);
+                    if (L.width == 16) node_grouped<16, 1><<<ctas, tch::THREADS, tch::Smem<16>::BYTES, s>>>(ne, L.n, L.blocks);
                 } else {
-                    if (L.width == 8) node_grouped<8, 2><<<(unsigned)L.blocks, merkle::TPB, 0, s>>>(ne, L.n);
-                    if (L.width == 12) node_grouped<12, 2><<<(unsigned)L.blocks, merkle::TPB, 0, s>>>(ne, L.n);
-                    if (L.width == 16) node_grouped<16, 2><<<(unsigned)L.blocks, merkle::TPB, 0, s>>>(ne, L.n);
+                    if (L.width == 8) node_grouped<8, 2><<<ctas, tch::THREADS, tch::Smem<8>::BYTES, s>>>(ne, L.n, L.blocks);
+                    if (L.width == 12) node_grouped<12, 2><<<ctas, tch::THREADS, tch::Smem<12>::BYTES, s>>>(ne, L.n, L.blocks);
+                    if (L.width == 16) node_grouped<16, 2><<<ctas, tch::THREADS, tch::Smem<16>::BYTES, s>>>(ne, L.n, L.blocks);
                 }
                 break;
             }

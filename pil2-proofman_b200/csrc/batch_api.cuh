@@ -28,6 +28,7 @@ static int batch_kernel_attrs()
                                 (NTT_TILE_MAX + NTT_TILE_MAX / 16) * 8),
            "pass_grouped smem attribute");
         CK(batch::set_grouped_fixed_attrs(), "pass_fixed_grouped smem attributes");
+        CK(batch::set_grouped_hash_attrs(), "grouped hashing smem attributes");
         done[dev] = true;
     }
     return B200_OK;

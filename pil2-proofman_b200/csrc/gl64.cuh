@@ -242,6 +242,63 @@ __device__ __forceinline__ uint64_t mul_pow2(uint64_t x)
     return sub_c(w, mk64(u1, u2));
 }
 
+// Montgomery reduction: (r3:r2:r1:r0) * 2^-64 mod p, loose, of any 128-bit value hi * 2^64 + lo.  p = 1 - 2^32 + 2^64, so
+// lo * p^-1 mod 2^64 is a = lo + (lo << 32), its product with p has the high half b = a - (a >> 32) - e (e the carry of
+// that sum), and the result is hi - b, plus p on a borrow (b < p, so one fold suffices).  With a1 = r1 + r0 that is
+// (hi + a1 + e) - (a1:r0): nine additions and no multiplication, where reduce128 takes eight and a product by 2^32 - 1.
+// SHORT leaves one out: the caller's hi is at most 2^64 - 2^32, so hi + a1 + e does not carry.
+template <bool SHORT>
+__device__ __forceinline__ uint64_t mont_reduce(uint32_t r0, uint32_t r1, uint32_t r2, uint32_t r3)
+{
+    uint32_t z0, z1, m;
+    if (SHORT)
+        asm("{\n\t.reg .u32 a;\n\t"
+            "add.cc.u32  a, %3, %4;\n\t"
+            "addc.cc.u32 %0, %5, a;\n\t"
+            "addc.u32    %1, %6, 0;\n\t"
+            "sub.cc.u32  %0, %0, %3;\n\t"
+            "subc.cc.u32 %1, %1, a;\n\t"
+            "subc.u32    %2, 0, 0;\n\t}"
+            : "=&r"(z0), "=&r"(z1), "=&r"(m)
+            : "r"(r0), "r"(r1), "r"(r2), "r"(r3));
+    else
+        asm("{\n\t.reg .u32 a, c;\n\t"
+            "add.cc.u32  a, %3, %4;\n\t"
+            "addc.cc.u32 %0, %5, a;\n\t"
+            "addc.cc.u32 %1, %6, 0;\n\t"
+            "addc.u32    c, 0, 0;\n\t"
+            "sub.cc.u32  %0, %0, %3;\n\t"
+            "subc.cc.u32 %1, %1, a;\n\t"
+            "subc.u32    %2, c, 0;\n\t}"
+            : "=&r"(z0), "=&r"(z1), "=&r"(m)
+            : "r"(r0), "r"(r1), "r"(r2), "r"(r3));
+    return mk64(z0, z1) - (uint64_t)m;  // m = 2^32 - 1 on a borrow
+}
+
+// a * b * 2^-64, loose
+__device__ __forceinline__ uint64_t mont_mul(uint64_t a, uint64_t b)
+{
+    uint32_t r0, r1, r2, r3;
+    mul128(a, b, r0, r1, r2, r3);
+    return mont_reduce<false>(r0, r1, r2, r3);
+}
+
+// a * b * 2^-64 for b canonical (then the result is canonical: hi < p) or both at most MONT_MAX (then so is the result)
+constexpr uint64_t MONT_MAX = 0xFFFFFFFF80000000ULL;  // 2^64 - 2^31, the largest x with x^2 >> 64 <= 2^64 - 2^32
+__device__ __forceinline__ uint64_t mont_mul_c(uint64_t a, uint64_t b)
+{
+    uint32_t r0, r1, r2, r3;
+    mul128(a, b, r0, r1, r2, r3);
+    return mont_reduce<true>(r0, r1, r2, r3);
+}
+
+// x^7 * 2^(-64 * 6) for x at most MONT_MAX
+__device__ __forceinline__ uint64_t mont_pow7(uint64_t x)
+{
+    const uint64_t x2 = mont_mul_c(x, x), x3 = mont_mul_c(x, x2), x4 = mont_mul_c(x2, x2);
+    return mont_mul_c(x3, x4);
+}
+
 // x^7 = x^3 * x^4, the Poseidon2 S-box (poseidon2_goldilocks.hpp:147-155)
 __device__ __forceinline__ uint64_t pow7(uint64_t x)
 {
@@ -315,6 +372,8 @@ static inline uint64_t pow(uint64_t b, uint64_t e)
     }
     return acc;
 }
+// a times 2^64: the other factor of gl::mont_mul
+static inline uint64_t mont(uint64_t a) { return mul(a, GL_EPS); }
 static inline uint64_t inv(uint64_t a) { return pow(a, GL_P - 2); }
 // W[k]: the reference's 2^k-th roots of unity (goldilocks_base_field.cpp:11-44), which are
 // W[32] = 0x64fdd1a46201e246 squared down: W[k] = W[k+1]^2.

@@ -19,14 +19,15 @@
 #include "poseidon1.cuh"
 #include "poseidon2.cuh"
 #include "prof.cuh"
+#include "tc_hash.cuh"
 
 namespace merkle {
 
-constexpr int TPB = 128;  // threads per CTA of the hashing kernels (one row / node / state each)
+constexpr int TPB = 128;  // threads per CTA of permute_kernel (one state each)
 
-// Hash family (the reference's set_hash_family): 1 = Poseidon1, 2 = Poseidon2.  Both use the same
-// sponge and tree; the Poseidon1 permutation needs a second W x TPB shared area for its matrix
-// steps, right after the state area.
+// Hash family (the reference's set_hash_family): 1 = Poseidon1, 2 = Poseidon2.  Both use the same sponge and
+// tree.  permute_kernel, which returns every word of a state, runs the one-thread-a-state permutations; the
+// Poseidon1 one needs a second W x TPB shared area for its matrix steps, right after the state area.
 template <int FAM>
 struct Family {
     static constexpr int SMEM_AREAS = FAM == 1 ? 2 : 1;
@@ -45,104 +46,39 @@ __device__ __forceinline__ void permute_fam(uint64_t *st)
         p2::permute_smem<W, TPB>(st);
 }
 
-// Digest i of a level sits at base + 4*i words, so every digest has the base's alignment.  A
-// 16-byte aligned base takes two 16-byte stores / loads per digest, any other base (a tree at an odd
-// word offset of a caller's buffer) four 8-byte ones; the test is uniform across the launch.
-__device__ __forceinline__ void store_digest(uint64_t *d, const uint64_t *st)
+// Row sponges of `nrows` rows, 128-row tiles over the groups of every CTA (tc_hash.cuh), tile t to CTA t mod the
+// grid first so that few tiles spread over the SMs.  Against one thread a row with the state in shared memory and
+// every layer on the integer pipes, 2^20 rows (B200): Poseidon2 W16 x 256 columns 24.6 -> 16.4 ms (937 -> 1403 M
+// permutations/s), W12 x 128 13.9 -> 9.8, W8 x 64 9.6 -> 7.5; Poseidon1 W16 39.0 -> 16.3, W12 19.4 -> 9.7, W8 12.5 -> 7.4.
+template <int W, int FAM = 2>
+__global__ void __launch_bounds__(tch::THREADS, 1) leaf_hash_kernel(uint64_t *__restrict__ digests,
+                                                                    const uint64_t *__restrict__ src, uint64_t rs,
+                                                                    uint64_t cs, uint64_t ncols, uint64_t nrows,
+                                                                    int resume)
 {
-    const uint64_t a = gl::canon(st[0]), b = gl::canon(st[TPB]), c = gl::canon(st[2 * TPB]), e = gl::canon(st[3 * TPB]);
-    if ((reinterpret_cast<uintptr_t>(d) & 15) == 0) {
-        reinterpret_cast<ulonglong2 *>(d)[0] = make_ulonglong2(a, b);
-        reinterpret_cast<ulonglong2 *>(d)[1] = make_ulonglong2(c, e);
-    } else {
-        d[0] = a;
-        d[1] = b;
-        d[2] = c;
-        d[3] = e;
-    }
+    extern __shared__ __align__(128) uint8_t tc_sm[];
+    __shared__ tch::Shared sh;
+    tch::Group<W, FAM> G;
+    G.setup(tc_sm, sh);
+    const uint64_t tiles = (nrows + 127) / 128;
+    for (uint64_t t = blockIdx.x + (uint64_t)gridDim.x * G.id; t < tiles; t += (uint64_t)gridDim.x * tch::GROUPS)
+        tch::leaf_tile(G, digests, src, rs, cs, ncols, nrows, t, resume != 0);
+    G.finish(sh);
 }
 
-// Sponge of one row; st = this thread's state slot in a W x TPB shared array.
+// One tree level of `parents` parents.
 template <int W, int FAM = 2>
-__device__ __forceinline__ void leaf_row(uint64_t *st, uint64_t *__restrict__ digests,
-                                         const uint64_t *__restrict__ src, uint64_t rs, uint64_t cs, uint64_t ncols,
-                                         uint64_t row)
+__global__ void __launch_bounds__(tch::THREADS, 1) node_kernel(uint64_t *__restrict__ level, uint64_t pending, uint64_t pad,
+                                                               uint64_t parents, uint64_t *__restrict__ out)
 {
-    constexpr int RATE = W - 4;
-#pragma unroll
-    for (int i = 0; i < W; i++) st[i * TPB] = 0;
-    const uint64_t *p = src + row * rs;
-    for (uint64_t done = 0; done < ncols; done += RATE) {
-        const uint64_t n = ncols - done;
-        if (done != 0) {
-#pragma unroll
-            for (int j = 0; j < 4; j++) st[(RATE + j) * TPB] = st[j * TPB];
-        }
-        if (n >= (uint64_t)RATE) {
-#pragma unroll
-            for (int i = 0; i < RATE; i++) st[i * TPB] = __ldg(p + (done + i) * cs);
-        } else {
-#pragma unroll
-            for (int i = 0; i < RATE; i++) st[i * TPB] = (uint64_t)i < n ? __ldg(p + (done + i) * cs) : 0ull;
-        }
-        permute_fam<W, FAM>(st);
-    }
-    // ncols == 0 leaves the state zeroed: the zero digest
-    store_digest(digests + row * 4, st);
-}
-
-template <int W, int FAM = 2>
-__global__ void __launch_bounds__(TPB, Family<FAM>::MIN_CTAS) leaf_hash_kernel(uint64_t *__restrict__ digests,
-                                                        const uint64_t *__restrict__ src, uint64_t rs,
-                                                        uint64_t cs, uint64_t ncols, uint64_t nrows)
-{
-    __shared__ uint64_t sm[Family<FAM>::SMEM_AREAS * W * TPB];
-    const uint64_t row = (uint64_t)blockIdx.x * TPB + threadIdx.x;
-    if (row < nrows) leaf_row<W, FAM>(sm + threadIdx.x, digests, src, rs, cs, ncols, row);
-}
-
-// Parent i of one tree level: `pending` child digests at `level`, `pad` zero digests written
-// after them (by the last parent), parents written to `out` (= level + 4*(pending + pad)).
-template <int W, int FAM = 2>
-__device__ __forceinline__ void node_one(uint64_t *st, uint64_t *__restrict__ level, uint64_t pending, uint64_t pad,
-                                         uint64_t parents, uint64_t *__restrict__ out, uint64_t i)
-{
-    constexpr int ARITY = W / 4;
-#pragma unroll
-    for (int c = 0; c < ARITY; c++) {
-        const uint64_t child = i * ARITY + c;
-        if (child < pending) {
-            const uint64_t *q = level + child * 4;
-            if ((reinterpret_cast<uintptr_t>(q) & 15) == 0) {
-                const ulonglong2 v0 = reinterpret_cast<const ulonglong2 *>(q)[0],
-                                 v1 = reinterpret_cast<const ulonglong2 *>(q)[1];
-                st[(4 * c + 0) * TPB] = v0.x;
-                st[(4 * c + 1) * TPB] = v0.y;
-                st[(4 * c + 2) * TPB] = v1.x;
-                st[(4 * c + 3) * TPB] = v1.y;
-            } else {
-#pragma unroll
-                for (int j = 0; j < 4; j++) st[(4 * c + j) * TPB] = q[j];
-            }
-        } else {
-#pragma unroll
-            for (int j = 0; j < 4; j++) st[(4 * c + j) * TPB] = 0;
-        }
-    }
-    if (i == parents - 1) {
-        for (uint64_t z = 0; z < pad * 4; z++) level[pending * 4 + z] = 0;
-    }
-    permute_fam<W, FAM>(st);
-    store_digest(out + i * 4, st);
-}
-
-template <int W, int FAM = 2>
-__global__ void __launch_bounds__(TPB, Family<FAM>::MIN_CTAS) node_kernel(uint64_t *__restrict__ level, uint64_t pending, uint64_t pad,
-                                                   uint64_t parents, uint64_t *__restrict__ out)
-{
-    __shared__ uint64_t sm[Family<FAM>::SMEM_AREAS * W * TPB];
-    const uint64_t i = (uint64_t)blockIdx.x * TPB + threadIdx.x;
-    if (i < parents) node_one<W, FAM>(sm + threadIdx.x, level, pending, pad, parents, out, i);
+    extern __shared__ __align__(128) uint8_t tc_sm[];
+    __shared__ tch::Shared sh;
+    tch::Group<W, FAM> G;
+    G.setup(tc_sm, sh);
+    const uint64_t tiles = (parents + 127) / 128;
+    for (uint64_t t = blockIdx.x + (uint64_t)gridDim.x * G.id; t < tiles; t += (uint64_t)gridDim.x * tch::GROUPS)
+        tch::node_tile(G, level, pending, pad, parents, out, t);
+    G.finish(sh);
 }
 
 // Whole permutations of n independent states (permute / permuteTrunc checks).
@@ -172,19 +108,17 @@ inline uint64_t tree_num_elements(uint64_t nrows, uint64_t arity)
     return total * 4;
 }
 
-// Below this many states per launch the one-thread-per-state hashing kernels leave the GPU idle
-// and take the latency of one whole permutation per thread (~40 us for Poseidon2 W16); the
-// cooperative kernels (coop.cuh, one state per 16 lanes) take it instead.
+// Below this many states per launch the tiled kernels leave most of the GPU idle and take the latency of whole
+// permutations (~20 us each); the cooperative kernels (coop.cuh, one state per 16 lanes) take it instead.
 constexpr uint64_t COOP_MAX_STATES = 8192;
 
 // Every tree level above `nrows` leaf digests already at the start of d_tree, on `stream`.
-// Levels of more than COOP_MAX_STATES parents one thread per parent, smaller ones cooperatively,
+// Levels of more than COOP_MAX_STATES parents in 128-parent tiles, smaller ones cooperatively,
 // and the last levels (<= coop::TAIL_THREADS / G parents) in one launch; both hash families.
 template <int W, int FAM = 2>
 cudaError_t build_levels(uint64_t *d_tree, uint64_t nrows, cudaStream_t stream)
 {
     constexpr uint64_t ARITY = W / 4;
-    const unsigned tpb = TPB;
     prof::Scope ps(prof::TREE_LEVELS, stream);
     uint64_t pending = nrows, base = 0;
     while (pending > 1) {
@@ -209,12 +143,23 @@ cudaError_t build_levels(uint64_t *d_tree, uint64_t nrows, cudaStream_t stream)
                 continue;
             }
         }
-        node_kernel<W, FAM><<<(unsigned)((parents + tpb - 1) / tpb), tpb, 0, stream>>>(lvl, pending, pad, parents,
-                                                                                   lvl + (pending + pad) * 4);
+        node_kernel<W, FAM><<<tch::grid((parents + 127) / 128), tch::THREADS, tch::Smem<W>::BYTES, stream>>>(
+            lvl, pending, pad, parents, lvl + (pending + pad) * 4);
         prof::count();
         base += (pending + pad) * 4;
         pending = parents;
     }
+    return cudaGetLastError();
+}
+
+// Row sponges into `digests` (resume: continuing from the words there), on `stream`.
+template <int W, int FAM = 2>
+cudaError_t hash_rows(uint64_t *digests, const uint64_t *src, uint64_t rs, uint64_t cs, uint64_t ncols, uint64_t nrows,
+                      bool resume, cudaStream_t stream)
+{
+    leaf_hash_kernel<W, FAM><<<tch::grid((nrows + 127) / 128), tch::THREADS, tch::Smem<W>::BYTES, stream>>>(
+        digests, src, rs, cs, ncols, nrows, resume ? 1 : 0);
+    prof::count();
     return cudaGetLastError();
 }
 
@@ -224,18 +169,17 @@ cudaError_t build_tree(uint64_t *d_tree, const uint64_t *d_src, uint64_t rs, uin
                        uint64_t nrows, cudaStream_t stream)
 {
     if (nrows == 0) return cudaSuccess;
-    const unsigned tpb = TPB;
     {
         prof::Scope ps(prof::LEAF_HASH, stream);
         if (nrows <= COOP_MAX_STATES) {
             const uint64_t threads = nrows * coop::Tab<W>::G;
             coop::leaf_coop_kernel<W, FAM><<<(unsigned)((threads + coop::CTA_THREADS - 1) / coop::CTA_THREADS),
                                              coop::CTA_THREADS, 0, stream>>>(d_tree, d_src, rs, cs, ncols, nrows);
+            prof::count();
         } else {
-            leaf_hash_kernel<W, FAM><<<(unsigned)((nrows + tpb - 1) / tpb), tpb, 0, stream>>>(d_tree, d_src, rs, cs,
-                                                                                           ncols, nrows);
+            const cudaError_t e = hash_rows<W, FAM>(d_tree, d_src, rs, cs, ncols, nrows, false, stream);
+            if (e != cudaSuccess) return e;
         }
-        prof::count();
     }
     return build_levels<W, FAM>(d_tree, nrows, stream);
 }
@@ -258,6 +202,28 @@ inline cudaError_t build_tree_arity(uint64_t arity, uint64_t *d_tree, const uint
     case 4: return build_tree<16>(d_tree, d_src, rs, cs, ncols, nrows, stream);
     default: return cudaErrorInvalidValue;
     }
+}
+
+// tables and kernel attributes of the current device
+template <int W, int FAM>
+inline cudaError_t set_attrs()
+{
+    const cudaError_t e = cudaFuncSetAttribute(leaf_hash_kernel<W, FAM>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               tch::Smem<W>::BYTES);
+    if (e != cudaSuccess) return e;
+    return cudaFuncSetAttribute(node_kernel<W, FAM>, cudaFuncAttributeMaxDynamicSharedMemorySize, tch::Smem<W>::BYTES);
+}
+
+inline cudaError_t init()
+{
+    cudaError_t e = tch::init_tables();
+    if (e == cudaSuccess) e = set_attrs<8, 1>();
+    if (e == cudaSuccess) e = set_attrs<8, 2>();
+    if (e == cudaSuccess) e = set_attrs<12, 1>();
+    if (e == cudaSuccess) e = set_attrs<12, 2>();
+    if (e == cudaSuccess) e = set_attrs<16, 1>();
+    if (e == cudaSuccess) e = set_attrs<16, 2>();
+    return e;
 }
 
 }  // namespace merkle

@@ -54,6 +54,7 @@ static int ensure_init_current()
                             (NTT_TILE_MAX + NTT_TILE_MAX / 16) * 8),
        "pass16_kernel smem attribute");
     CK(ntt::set_fixed_attrs(), "pass_fixed_kernel smem attributes");
+    CK(merkle::init(), "hash tables");
     g_init_done[dev] = true;
     return B200_OK;
 }
@@ -281,7 +282,7 @@ extern "C" const char *b200_kernel_names(void)
     return "pass16_kernel\ntranspose_kernel\ntranspose_tma_kernel\nleaf_hash_kernel\nnode_kernel\npermute_kernel\nlde_rows_kernel\n"
            "fill_kernel\nimad_probe_kernel\ntranspose_grouped\npass_grouped\nleaf_persistent\n"
            "node_grouped\ngather_roots\npass_fixed_kernel\nopenings_kernel\nbitfield_unpack_kernel\n"
-           "unpack_range_kernel\nabsorb_kernel\npass_fixed_grouped\nnode_coop_kernel\ntree_tail_kernel\n"
+           "unpack_range_kernel\npass_fixed_grouped\nnode_coop_kernel\ntree_tail_kernel\n"
            "leaf_coop_kernel\n";
 }
 
@@ -668,7 +669,7 @@ struct PipeBuffers {
 //
 // With `idle` (nothing else runs on the device, so the copy is exposed), an arity-4 commit hashes
 // its rows while the later column blocks are still crossing: the row sponge in 12-column chunks
-// (stream::absorb_kernel, the 4-word state carried in tree level 0), each chunk as soon as its
+// (merkle::hash_rows, the 4-word state carried in tree level 0), each chunk as soon as its
 // columns are extended.  Same sponge, same digests.
 static int pipelined_commit(const uint64_t *trace, uint64_t nBits, uint64_t nBitsExt, uint64_t nCols, uint64_t arity,
                             int fam, const PipeBuffers &pb, cudaStream_t copy, cudaStream_t comp,
@@ -714,19 +715,15 @@ static int pipelined_commit(const uint64_t *trace, uint64_t nBits, uint64_t nBit
         if (chunked) {
             const uint64_t avail = k + 1 == nblk ? nCols : c0 + cb;  // columns extended so far
             prof::Scope ps(prof::LEAF_HASH, comp);
-            for (; next_chunk * stream::RATE < nCols; next_chunk++) {
-                const uint64_t a0 = next_chunk * stream::RATE;
-                const uint32_t cc = (uint32_t)std::min<uint64_t>(stream::RATE, nCols - a0);
-                if (a0 + cc > avail) break;
-                const unsigned grid = (unsigned)((NExt + merkle::TPB - 1) / merkle::TPB);
-                if (fam == 1)
-                    stream::absorb_kernel<1><<<grid, merkle::TPB, 0, comp>>>(pb.tree, pb.lde + a0 * NExt, cc,
-                                                                             next_chunk == 0, NExt);
-                else
-                    stream::absorb_kernel<2><<<grid, merkle::TPB, 0, comp>>>(pb.tree, pb.lde + a0 * NExt, cc,
-                                                                             next_chunk == 0, NExt);
-                prof::count();
-                CK(cudaGetLastError(), "absorb");
+            // every whole 12-column chunk that has been extended (and the last, shorter one), in one launch
+            const uint64_t a0 = next_chunk * stream::RATE;
+            const uint64_t upto = avail == nCols ? nCols : avail / stream::RATE * stream::RATE;
+            if (upto > a0) {
+                const uint64_t *src = pb.lde + a0 * NExt;
+                CK(fam == 1 ? (merkle::hash_rows<16, 1>(pb.tree, src, 1, NExt, upto - a0, NExt, a0 != 0, comp))
+                            : (merkle::hash_rows<16, 2>(pb.tree, src, 1, NExt, upto - a0, NExt, a0 != 0, comp)),
+                   "absorb");
+                next_chunk = upto / stream::RATE;
             }
         }
     }
@@ -1044,14 +1041,16 @@ extern "C" uint64_t b200_launch_count(void) { return prof::g_launches.load(); }
 
 extern "C" int b200_set_transpose_tma(int on) { return ntt::transpose_tma_enabled().exchange(on ? 1 : 0); }
 
-// the TMA transposes' error flag on the current device (1: a tile copy did not land within the
-// kernel's wait bound), reset to 0
+// the bounded waits' error flags on the current device (1: a TMA tile copy or a tensor core product did not
+// complete within the kernel's wait bound), reset to 0
 extern "C" int b200_tma_wait_errors(void)
 {
-    int v = 0, zero = 0;
+    int v = 0, w = 0, zero = 0;
     if (cudaMemcpyFromSymbol(&v, g_tma_error, sizeof(int)) != cudaSuccess) return cuda_err(cudaGetLastError(), "flag");
+    if (cudaMemcpyFromSymbol(&w, g_tc_error, sizeof(int)) != cudaSuccess) return cuda_err(cudaGetLastError(), "flag");
     CK(cudaMemcpyToSymbol(g_tma_error, &zero, sizeof(int)), "flag reset");
-    return v;
+    CK(cudaMemcpyToSymbol(g_tc_error, &zero, sizeof(int)), "flag reset");
+    return v | w;
 }
 
 __global__ void __launch_bounds__(256) imad_probe_kernel(uint32_t *out, uint64_t iters, uint32_t seed)

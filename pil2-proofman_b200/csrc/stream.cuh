@@ -61,28 +61,6 @@ __global__ void __launch_bounds__(256) unpack_range_kernel(uint64_t *__restrict_
     }
 }
 
-// Absorb one chunk of cc <= RATE extended columns (column-major, stride nrows) into the carried
-// words `carry` (row-major, 4 per row = tree level 0).
-template <int FAM>
-__global__ void __launch_bounds__(merkle::TPB, merkle::Family<FAM>::MIN_CTAS) absorb_kernel(uint64_t *__restrict__ carry,
-                                                             const uint64_t *__restrict__ chunk, uint32_t cc,
-                                                             int first, uint64_t nrows)
-{
-    constexpr int W = 16;
-    constexpr int TPB = merkle::TPB;
-    __shared__ uint64_t sm[merkle::Family<FAM>::SMEM_AREAS * W * TPB];
-    const uint64_t row = (uint64_t)blockIdx.x * TPB + threadIdx.x;
-    if (row >= nrows) return;
-    uint64_t *st = sm + threadIdx.x;
-#pragma unroll
-    for (uint32_t i = 0; i < RATE; i++) st[i * TPB] = i < cc ? __ldg(chunk + (uint64_t)i * nrows + row) : 0ull;
-#pragma unroll
-    for (int i = 0; i < 4; i++) st[(RATE + i) * TPB] = first ? 0ull : carry[row * 4 + i];
-    merkle::permute_fam<W, FAM>(st);
-#pragma unroll
-    for (int i = 0; i < 4; i++) carry[row * 4 + i] = gl::canon(st[i * TPB]);
-}
-
 // Indexed witness: the instruction table on the device and the row header width; the slot's
 // width region then holds width | source << 32 per column (unpack::bitfield_unpack_kernel).
 struct Indexed {
@@ -114,10 +92,8 @@ inline cudaError_t run(uint64_t *slot, const Layout &l, uint64_t nBits, uint64_t
         prof::count();
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
         if ((e = ntt::lde(chunk, scr, false, (uint32_t)nBits, (uint32_t)nBitsExt, cc, scr, s)) != cudaSuccess) return e;
-        absorb_kernel<FAM><<<(unsigned)((NExt + merkle::TPB - 1) / merkle::TPB), merkle::TPB, 0, s>>>(
-            tree, chunk, cc, c0 == 0, NExt);
-        prof::count();
-        if ((e = cudaGetLastError()) != cudaSuccess) return e;
+        // the chunk's columns are one more block of every row's sponge, its carried words in tree level 0
+        if ((e = merkle::hash_rows<16, FAM>(tree, chunk, 1, NExt, cc, NExt, c0 != 0, s)) != cudaSuccess) return e;
     }
     return merkle::build_levels<16, FAM>(tree, NExt, s);
 }

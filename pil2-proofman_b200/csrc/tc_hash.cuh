@@ -1,0 +1,458 @@
+// Poseidon permutations with the linear layers on the tensor cores (8-bit integer tcgen05.mma).
+//
+// The tables of tc_tables.h turn every linear layer (the external / MDS layers of the full rounds, and all
+// of the partial rounds but their S-boxes) into products of a state's bytes with a constant byte matrix.
+// One group of 256 threads owns 128 states: the states' bytes are the 128 rows of the left operand in shared
+// memory (16-byte piece c of row r at c * 2048 + r * 16, so a thread's 16-byte accesses are conflict-free and
+// a state word is stored as it is), the accumulators are the 128 lanes of tensor memory, and a thread reads
+// its row's columns back and joins them to 64-bit words (join_word).
+//
+// What bounds it: the S-boxes' integer products (150 x^7 a width-16 permutation, at 0.85 clocks an SM each 128 of
+// the 207 clocks a permutation takes on a B200; IMAD.WIDE issues 25 lanes a clock and SM).  The tensor pipe is 12 %
+// busy, so no product is shaped for it: every layer goes through, also those with small coefficients, because
+// joining eight columns costs a third of the 128-bit sums that it replaces.  The S-boxes and joins run in
+// Montgomery form because that reduction needs no multiplication (gl64.cuh).
+//
+// A CTA is four groups, one CTA an SM: the tables take 106 KB of shared memory at width 16, each group 28 KB and a
+// quarter of the tensor memory (128 columns, a whole layer's).  Two threads share a row (each takes half its words, and
+// every other run of partial rounds), so 32 warps hide the barriers and latencies: one row of 128 rows x 40 columns
+// takes 20 % less than with one thread a row, large launches the same.  Groups run independently, so one's products
+// and barriers run under the others' S-boxes.
+#pragma once
+#include "gl64.cuh"
+#include "tc_tables.h"
+
+__device__ int g_tc_error;  // set when a product did not complete within the wait bound
+
+// Table bytes and constants by [family - 1][width / 4 - 2], uploaded once per device.
+__device__ __align__(16) uint8_t g_tc_tab[2][3][tch::MAX_BYTES];
+__constant__ tch::Consts c_tc[2][3];
+
+namespace tch {
+
+constexpr int GROUPS = 4, SPLIT = 2, STEP = 2, GTHREADS = 128 * SPLIT, THREADS = GTHREADS * GROUPS;
+constexpr uint32_t GROUP_COLS = 512 / GROUPS;  // tensor memory columns of a group
+constexpr uint32_t WAIT_LIMIT = 1u << 20;      // try_wait rounds before a thread gives up
+
+template <int W>
+struct Smem {
+    static constexpr int GROUP = (Shape<W>::CHX + YCH) * 2048;  // state rows and a block's y rows
+    static constexpr int BYTES = Shape<W>::BYTES + GROUPS * GROUP;
+};
+
+__device__ __forceinline__ uint32_t smem_addr(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
+
+// Shared-memory matrix descriptor, no swizzle: 8-row x 16-byte cores, `lbo` bytes between cores along K,
+// 128 bytes between cores along the rows.
+__device__ __forceinline__ uint64_t matrix_desc(uint32_t addr, uint32_t lbo)
+{
+    return (uint64_t)((addr & 0x3FFFFu) >> 4) | ((uint64_t)(lbo >> 4) << 16) | ((uint64_t)(128 >> 4) << 32) | (1ull << 46);
+}
+
+// u8 x u8 -> s32, 128 rows, n columns
+__host__ __device__ constexpr uint32_t instr_desc(uint32_t n) { return (2u << 4) | ((n >> 3) << 17) | ((128u >> 4) << 24); }
+
+__device__ __forceinline__ void mma_i8(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, bool accumulate)
+{
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}" ::"r"(d),
+        "l"(a), "l"(b), "r"(idesc), "r"((uint32_t)accumulate)
+        : "memory");
+}
+
+// 16 columns (two words) of this thread's row
+__device__ __forceinline__ void ld_cols16(uint32_t (&r)[16], uint32_t t)
+{
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n\t"
+        "tcgen05.wait::ld.sync.aligned;"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+        : "r"(t)
+        : "memory");
+}
+
+__device__ __forceinline__ void sts128(uint32_t a, uint64_t x, uint64_t y)
+{
+    asm volatile("st.shared.v2.b64 [%0], {%1, %2};" ::"r"(a), "l"(x), "l"(y) : "memory");
+}
+
+// 160-bit little-endian value
+struct Wide {
+    uint32_t w[5];
+};
+
+// Column pairs: t_i = col[2i] + 256 col[2i+1] < 2^31 (check_bounds), the word is sum_i t_i 2^(16 i).
+__device__ __forceinline__ void pairs(const uint32_t *col, uint32_t (&t)[4])
+{
+#pragma unroll
+    for (int i = 0; i < 4; i++) t[i] = col[2 * i] + (col[2 * i + 1] << 8);
+}
+
+// sum_i t_i 2^(16 i) + c in 96 bits
+__device__ __forceinline__ void join96(const uint32_t *col, uint64_t c, uint32_t &w0, uint32_t &w1, uint32_t &w2)
+{
+    uint32_t t[4];
+    pairs(col, t);
+    const uint64_t lo = (uint64_t)t[1] * 65536u + t[0], hi = (uint64_t)t[3] * 65536u + t[2];
+    asm("add.cc.u32  %0, %3, %7;\n\t"
+        "addc.cc.u32 %1, %4, %8;\n\t"
+        "addc.u32    %2, %6, 0;\n\t"
+        "add.cc.u32  %1, %1, %5;\n\t"
+        "addc.u32    %2, %2, 0;\n\t"
+        : "=&r"(w0), "=&r"(w1), "=&r"(w2)
+        : "r"(gl::lo32(lo)), "r"(gl::hi32(lo)), "r"(gl::lo32(hi)), "r"(gl::hi32(hi)), "r"(gl::lo32(c)), "r"(gl::hi32(c)));
+}
+
+// (sum_i t_i 2^(16 i)) 2^-32 + c, loose.  With x0 the sum's low word, one Montgomery step by 32 bits is
+// (sum - x0 p) / 2^32 = sum >> 32 + x0 - x0 2^32; c < 2^64 - 2^50 leaves room for the rest, so only the last
+// subtraction can wrap, once, and the result is at most gl::MONT_MAX.
+__device__ __forceinline__ uint64_t join_word(const uint32_t *col, uint64_t c)
+{
+    uint32_t t[4], x0, u;
+    pairs(col, t);
+    asm("add.cc.u32 %0, %2, %3;\n\t"
+        "addc.u32   %1, %4, %5;\n\t"
+        : "=&r"(x0), "=&r"(u)
+        : "r"(t[0]), "r"(t[1] << 16), "r"(t[2]), "r"(t[1] >> 16));
+    const uint64_t y = (uint64_t)t[3] * 65536u + c + u + x0;
+    uint32_t z1, m;
+    asm("sub.cc.u32 %0, %2, %3;\n\t"
+        "subc.u32   %1, 0, 0;\n\t"
+        : "=r"(z1), "=r"(m)
+        : "r"(gl::hi32(y)), "r"(x0));
+    return gl::mk64(gl::lo32(y), z1) - (uint64_t)m;
+}
+
+__device__ __forceinline__ void wide_mul_add(Wide &a, uint64_t x, uint64_t y)
+{
+    uint32_t r0, r1, r2, r3;
+    gl::mul128(x, y, r0, r1, r2, r3);
+    asm("add.cc.u32  %0, %0, %5;\n\t"
+        "addc.cc.u32 %1, %1, %6;\n\t"
+        "addc.cc.u32 %2, %2, %7;\n\t"
+        "addc.cc.u32 %3, %3, %8;\n\t"
+        "addc.u32    %4, %4, 0;\n\t"
+        : "+r"(a.w[0]), "+r"(a.w[1]), "+r"(a.w[2]), "+r"(a.w[3]), "+r"(a.w[4])
+        : "r"(r0), "r"(r1), "r"(r2), "r"(r3));
+}
+
+// 2^128 = -2^32 (mod p): reduce the low 128 bits, subtract w4 * 2^32 (< p)
+__device__ __forceinline__ uint64_t wide_reduce(const Wide &a)
+{
+    return gl::sub_c(gl::reduce128(a.w[0], a.w[1], a.w[2], a.w[3]), (uint64_t)a.w[4] << 32);
+}
+
+// Two canonical words to p: one 16-byte store where p is aligned for it (a tree may start at any word of a
+// caller's buffer), else two 8-byte ones.
+__device__ __forceinline__ void store_pair(uint64_t *p, const uint64_t (&v)[2])
+{
+    const uint64_t a = gl::canon(v[0]), b = gl::canon(v[1]);
+    if ((reinterpret_cast<uintptr_t>(p) & 15) == 0) {
+        *reinterpret_cast<ulonglong2 *>(p) = make_ulonglong2(a, b);
+    } else {
+        p[0] = a;
+        p[1] = b;
+    }
+}
+
+// A CTA's barriers and tensor memory address.
+struct Shared {
+    uint64_t mbar[GROUPS];
+    uint32_t tmem;
+};
+
+// A thread's view of its group.
+template <int W, int FAM>
+struct Group {
+    uint32_t row;      // shared address of this thread's row (piece 0)
+    uint32_t tab;      // shared address of the tables
+    uint32_t tmem;     // the group's first tensor memory column, this warp's lanes
+    uint32_t mbar;     // the group's barrier
+    uint32_t phase;
+    uint32_t id;       // group index
+    uint32_t half;     // this thread's share of the row's words
+    bool issuer, dead;
+
+    static constexpr int OUT = 4 / SPLIT;  // output words of a thread
+
+    static __device__ __forceinline__ const Consts &consts() { return c_tc[FAM - 1][W / 4 - 2]; }
+
+    __device__ __forceinline__ uint32_t word_addr(int i) const { return row + (uint32_t)(i >> 1) * 2048 + (i & 1) * 8; }
+
+    // Tables into shared memory, tensor memory, barriers.  All threads of the CTA.
+    __device__ __forceinline__ void setup(uint8_t *sm, Shared &sh)
+    {
+        const uint32_t warp = threadIdx.x >> 5;
+        const uint4 *src = reinterpret_cast<const uint4 *>(g_tc_tab[FAM - 1][W / 4 - 2]);
+        for (uint32_t i = threadIdx.x; i < (uint32_t)Shape<W>::BYTES / 16; i += THREADS)
+            reinterpret_cast<uint4 *>(sm)[i] = __ldg(src + i);
+        if (warp == 0) {
+            asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_addr(&sh.tmem))
+                         : "memory");
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+        }
+        if (threadIdx.x < GROUPS)
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(sh.mbar + threadIdx.x)) : "memory");
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        __syncthreads();
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        id = threadIdx.x / GTHREADS;
+        half = (threadIdx.x >> 7) & (SPLIT - 1);
+        const uint32_t r = threadIdx.x & 127;
+        tab = smem_addr(sm);
+        row = tab + Shape<W>::BYTES + id * Smem<W>::GROUP + r * 16;
+        tmem = sh.tmem + id * GROUP_COLS + ((warp & 3) << 21);
+        mbar = smem_addr(sh.mbar + id);
+        phase = 0;
+        issuer = (threadIdx.x & (GTHREADS - 1)) == 0;
+        dead = false;
+    }
+
+    // barrier of the group's threads
+    __device__ __forceinline__ void sync() const { asm volatile("bar.sync %0, %1;" ::"r"(id + 1), "n"(GTHREADS) : "memory"); }
+
+    __device__ __forceinline__ bool wait(uint32_t parity)
+    {
+        for (uint32_t i = 0; i < WAIT_LIMIT; i++) {
+            uint32_t done;
+            asm volatile(
+                "{\n\t.reg .pred p;\n\t"
+                "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+                "selp.u32 %0, 1, 0, p;\n\t}"
+                : "=r"(done)
+                : "r"(mbar), "r"(parity)
+                : "memory");
+            if (done) return true;
+        }
+        return false;
+    }
+
+    // The group's rows times a table of K bytes (K / 32 steps of 32) whose pieces hold `ld` columns, the first
+    // n of them into the group's tensor memory.  Ends with the columns readable.  If the product does not
+    // complete within the wait bound the thread flags the error and stops waiting (its words are then wrong).
+    __device__ __forceinline__ void product(uint32_t off, uint32_t ksteps, uint32_t ld, uint32_t idesc)
+    {
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        sync();
+        if (issuer && !dead) {
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            uint64_t a = matrix_desc(row, 2048), b = matrix_desc(tab + off, ld * 16);
+            for (uint32_t k = 0; k < ksteps; k++) {
+                mma_i8(tmem, a, b, idesc, k != 0);
+                a += 2 * 2048 / 16;
+                b += 2 * ld;
+            }
+            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(mbar) : "memory");
+        }
+        if (!dead && !wait(phase)) {
+            dead = true;
+            atomicExch(&g_tc_error, 1);
+        }
+        phase ^= 1;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    }
+
+    // Frees the tensor memory once every group is done with it.  All threads of the CTA.
+    __device__ __forceinline__ void finish(const Shared &sh)
+    {
+        if (dead) wait(phase ^ 1);  // give a late product one more bound to land
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        __syncthreads();
+        if (threadIdx.x < 32) {
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(sh.tmem));
+        }
+    }
+
+    // One run of N partial rounds: z_t from the product's words and the run's earlier y, y_t = z_t^7 into the
+    // block's y rows from y_{first}.  A chain, so one thread of a row does it: the first run's by one half of the
+    // threads, the second's by the other.
+    template <int N>
+    __device__ __forceinline__ void run(uint32_t off, uint32_t ksteps, int first, const uint64_t *kz, const uint64_t *q)
+    {
+        product(off, ksteps, NZ, instr_desc(NZ));
+        if (SPLIT == 2 && half != (N == RUN0 ? 0 : 1)) return;
+        uint64_t y[N];
+        uint32_t col[16];
+#pragma unroll
+        for (int t = 0; t < N; t++) {
+            if (t % 2 == 0) ld_cols16(col, tmem + 8 * t);
+            if (t == 0) {
+                y[0] = gl::mont_pow7(join_word(col, kz[0]));
+            } else {
+                Wide a;
+                join96(col + 8 * (t & 1), kz[t], a.w[0], a.w[1], a.w[2]);
+                a.w[3] = a.w[4] = 0;
+#pragma unroll
+                for (int u = 0; u < t; u++) wide_mul_add(a, y[u], q[t * (t - 1) / 2 + u]);
+                y[t] = gl::mont_pow7(gl::canon(wide_reduce(a)));
+            }
+        }
+#pragma unroll
+        for (int t = 0; t < N; t += 2) sts128(word_addr(W + first + t), y[t], t + 1 < N ? y[t + 1] : 0ull);
+    }
+
+    // The permutation of the states in the rows (Poseidon2: the state; Poseidon1: x^7 of the state plus the
+    // first constants, which has no layer before it).  out: words 0..3 of the result, loose.
+    __device__ __forceinline__ void permute(uint64_t (&out)[OUT])
+    {
+        typedef Shape<W> S;
+        const Consts &C = consts();
+#pragma unroll 1
+        for (int s = FAM == 2 ? 0 : 1; s < 9; s++) {
+            if (s == 4 || s == 5) {
+                const int b = s - 4;
+                run<RUN0>(S::OFF_Z0 + b * S::BLOCK, S::K_Z0 / 32, 0, C.z[b], C.q[b]);
+                run<RUN1>(S::OFF_Z1 + b * S::BLOCK, S::K_Z1 / 32, RUN0, C.z[b] + RUN0, C.q[b] + RUN0 * (RUN0 - 1) / 2);
+                product(S::OFF_U + b * S::BLOCK, S::K_U / 32, S::KX, instr_desc(S::KX));
+            } else {
+                product(S::OFF_L, S::KX / 32, S::KX, instr_desc(S::KX));
+            }
+            const uint64_t *k = C.lay[s];
+#pragma unroll 1
+            for (int i = 0; i < W / SPLIT; i += STEP) {
+                const int g = half * (W / SPLIT) + i;
+                uint32_t col[8 * STEP];
+                ld_cols16(col, tmem + 8 * g);
+                uint64_t x[STEP];
+#pragma unroll
+                for (int j = 0; j < STEP; j++) x[j] = join_word(col + 8 * j, k[g + j]);
+                if (s != 4) {
+#pragma unroll
+                    for (int j = 0; j < STEP; j++) x[j] = gl::mont_pow7(x[j]);
+                }
+#pragma unroll
+                for (int j = 0; j < STEP; j += 2) sts128(word_addr(g + j), x[j], x[j + 1]);
+            }
+        }
+        product(S::OFF_F, S::KX / 32, S::NF, instr_desc(S::NF));
+        uint32_t col[8 * OUT];
+        ld_cols16(col, tmem + 8 * OUT * half);
+#pragma unroll
+        for (int j = 0; j < OUT; j++) out[j] = join_word(col + 8 * j, 0);
+    }
+
+    // words g and g + 1 of a state into the rows (g even)
+    __device__ __forceinline__ void put2(int g, uint64_t a, uint64_t b) const
+    {
+        if (FAM == 1) {
+            const uint64_t *k = consts().lay[0];
+            a = gl::pow7(gl::add_c(a, k[g]));
+            b = gl::pow7(gl::add_c(b, k[g + 1]));
+        }
+        sts128(word_addr(g), a, b);
+    }
+};
+
+// Row sponge of up to 128 rows (capacity zeroed at the start; every block of RATE columns overwrites words
+// [0, RATE), zero past the last column, and carries words [0, 4) into the capacity; 0 columns give the zero digest:
+// poseidon2_goldilocks.cpp:42-77).  `resume`: the digests hold the four words of the blocks before.  Threads past the last
+// row hash it again and store nothing.
+template <int W, int FAM>
+__device__ __forceinline__ void leaf_tile(Group<W, FAM> &G, uint64_t *__restrict__ digests,
+                                          const uint64_t *__restrict__ src, uint64_t rs, uint64_t cs, uint64_t ncols,
+                                          uint64_t nrows, uint64_t tile, bool resume)
+{
+    constexpr int RATE = W - 4, MINE = RATE / SPLIT, OUT = Group<W, FAM>::OUT;
+    uint64_t row = tile * 128 + (threadIdx.x & 127);
+    const bool valid = row < nrows;
+    if (!valid) row = nrows - 1;
+    const int first = (int)G.half * MINE;
+    const uint64_t *p = src + row * rs;
+    uint64_t *d = digests + row * 4 + G.half * OUT;
+    uint64_t cap[OUT] = {};
+    if (resume) {
+#pragma unroll
+        for (int i = 0; i < OUT; i++) cap[i] = d[i];
+    }
+    for (uint64_t done = 0; done < ncols; done += RATE) {
+        const uint64_t at = done + first;
+        uint64_t v[MINE];
+#pragma unroll
+        for (int i = 0; i < MINE; i++) v[i] = at + i < ncols ? __ldg(p + (at + i) * cs) : 0ull;
+#pragma unroll
+        for (int i = 0; i < MINE; i += 2) G.put2(first + i, v[i], v[i + 1]);
+        G.put2(RATE + (int)G.half * OUT, cap[0], cap[1]);
+        G.permute(cap);
+    }
+    if (valid) store_pair(d, cap);
+}
+
+// Parents of up to 128 nodes of one tree level (poseidon2_goldilocks.cpp:129-175): `pending` child digests at
+// `level`, `pad` zero digests after them (written by the last parent), parents written to `out`; parent i hashes the
+// W words of its children, zero past `pending`.
+template <int W, int FAM>
+__device__ __forceinline__ void node_tile(Group<W, FAM> &G, uint64_t *__restrict__ level, uint64_t pending, uint64_t pad,
+                                          uint64_t parents, uint64_t *__restrict__ out, uint64_t tile)
+{
+    constexpr int MINE = W / SPLIT;
+    const uint64_t i = tile * 128 + (threadIdx.x & 127);
+    const uint64_t first = i * W + G.half * MINE, end = pending * 4;
+    if (i == parents - 1 && G.half == 0)
+        for (uint64_t z = 0; z < pad * 4; z++) level[end + z] = 0;
+    uint64_t v[MINE];
+    const uint64_t *q = level + first;
+    if ((reinterpret_cast<uintptr_t>(q) & 15) == 0 && first + MINE <= end) {
+#pragma unroll
+        for (int j = 0; j < MINE; j += 2) {
+            const ulonglong2 w = *reinterpret_cast<const ulonglong2 *>(q + j);
+            v[j] = w.x;
+            v[j + 1] = w.y;
+        }
+    } else {
+#pragma unroll
+        for (int j = 0; j < MINE; j++) v[j] = first + j < end ? q[j] : 0ull;
+    }
+#pragma unroll
+    for (int j = 0; j < MINE; j += 2) G.put2((int)G.half * MINE + j, v[j], v[j + 1]);
+    uint64_t o[2];
+    G.permute(o);
+    if (i < parents) store_pair(out + i * 4 + G.half * 2, o);
+}
+
+// ------------------------------------------------------------------ host side ----
+
+template <int W>
+inline cudaError_t upload(int fam)
+{
+    static uint8_t tab[MAX_BYTES];
+    Consts c;
+    build_tables<W>(fam, tab, c);
+    const size_t i = (size_t)(fam - 1) * 3 + (W / 4 - 2);
+    cudaError_t e = cudaMemcpyToSymbol(g_tc_tab, tab, Shape<W>::BYTES, i * MAX_BYTES);
+    if (e != cudaSuccess) return e;
+    return cudaMemcpyToSymbol(c_tc, &c, sizeof(c), i * sizeof(Consts));
+}
+
+template <int W>
+inline cudaError_t upload()
+{
+    const cudaError_t e = upload<W>(1);
+    return e != cudaSuccess ? e : upload<W>(2);
+}
+
+// the tables of every width and family on the current device
+inline cudaError_t init_tables()
+{
+    cudaError_t e;
+    if ((e = upload<8>()) != cudaSuccess) return e;
+    if ((e = upload<12>()) != cudaSuccess) return e;
+    return upload<16>();
+}
+
+// CTAs of a launch over `tiles` 128-row tiles: one an SM, no more than tiles
+inline unsigned grid(uint64_t tiles)
+{
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms < 1)
+        sms = 1;
+    return (unsigned)(tiles < (uint64_t)sms ? tiles : (uint64_t)sms);
+}
+
+}  // namespace tch

@@ -1,0 +1,57 @@
+"""The tensor core hashing kernels (tc_hash.cuh) against the oracle, above the cooperative kernels' range.
+
+Edges: one row into a new 128-row tile, one tile more than the resident groups (148 SMs x 4), sponges of no,
+one and more blocks with a full and a ragged last one, both strides, a tree at an odd word of its buffer
+(8-byte stores), words from 0 to 2^64 - 1, and a level whose last parent has missing children.
+Whole trees are compared, bit for bit.
+"""
+import numpy as np
+import pytest
+
+import oracle
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def dev(pkg):
+    torch = pytest.importorskip("torch")
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    pkg.init(0)
+    yield pkg, torch
+    pkg.set_native_hash_family(2)
+    assert pkg.load().b200_tma_wait_errors() == 0  # no bounded wait ran out
+
+
+# rows, columns in sponge blocks (blocks, extra columns)
+ROWS = [8193, 8320, 148 * 4 * 128 + 1]
+COLS = [(0, 0), (1, 0), (1, 1), (2, -1)]
+
+
+@pytest.mark.parametrize("family", [1, 2])
+@pytest.mark.parametrize("arity", [2, 3, 4])
+@pytest.mark.parametrize("nrows", ROWS)
+def test_tree_at_the_tiles_edges(dev, arity, family, nrows):
+    pkg, torch = dev
+    orc = oracle.Oracle(family=family)
+    pkg.set_native_hash_family(family)
+    rate = 4 * arity - 4
+    blocks, extra = COLS[(nrows + arity + family) % len(COLS)]
+    for k, (b, x) in enumerate([(blocks, extra), (1, 0)]):
+        ncols = b * rate + x
+        m = oracle.random_field((nrows, ncols), nrows + ncols + family)
+        if ncols:
+            m[0] = np.uint64(2**64 - 1)
+            m[-1] = np.uint64(oracle.P - 1)
+        exp = orc.merkletree(m % np.uint64(oracle.P), arity)
+        colmajor = k == 0
+        src = np.ascontiguousarray(m.T if colmajor else m)
+        d_src = torch.from_numpy((src if src.size else np.zeros(1, np.uint64)).view(np.int64)).cuda()
+        buf = torch.zeros(exp.size + 1, dtype=torch.int64, device="cuda")
+        tree = buf[k:k + exp.size]  # the second at an odd word
+        rs, cs = (1, nrows) if colmajor else (ncols, 1)
+        pkg.merkletree_device(tree, d_src, rs, cs, ncols, nrows, arity)
+        torch.cuda.synchronize()
+        bad = np.nonzero(tree.cpu().numpy().view(np.uint64) != exp)[0]
+        assert bad.size == 0, (nrows, ncols, arity, family, bad[:8])
