@@ -32,6 +32,8 @@
 #define NTT_TWLG 26   // inter-window twiddles: powers of w_{2^26}; transforms up to 2^26 points
 #define NTT_TILE_MAX 8192
 
+// Every table holds its factors times 2^64 (Montgomery form), so a product with gl::mont_mul is the plain
+// product of the element and the factor, and products of two factors stay in that form.
 __device__ uint64_t g_ntt_tw_lo_fwd[1 << 13];
 __device__ uint64_t g_ntt_tw_hi_fwd[1 << 13];
 __device__ uint64_t g_ntt_tw_lo_inv[1 << 13];
@@ -54,7 +56,7 @@ struct Pass {
     uint32_t post;            // POST_*
     uint32_t gshift;          // source index = ((dst position >> rep) << gshift) + goff
     uint64_t goff;
-    uint64_t scale;           // loads multiplied by this factor (0: no scaling)
+    uint64_t scale;           // loads multiplied by this factor, times 2^64 (0: no scaling)
 };
 
 __device__ __forceinline__ uint32_t brev_bits(uint32_t x, uint32_t bits)
@@ -66,7 +68,7 @@ __device__ __forceinline__ uint64_t big_twiddle(uint64_t e, bool inv)
 {
     const uint64_t *lo = inv ? g_ntt_tw_lo_inv : g_ntt_tw_lo_fwd;
     const uint64_t *hi = inv ? g_ntt_tw_hi_inv : g_ntt_tw_hi_fwd;
-    return gl::mul(__ldg(lo + (e & 8191)), __ldg(hi + (e >> 13)));
+    return gl::mont_mul_c(__ldg(lo + (e & 8191)), __ldg(hi + (e >> 13)));
 }
 
 // ---------------------------------------------------------------------------------
@@ -104,10 +106,10 @@ __device__ __forceinline__ uint64_t mul_root16(uint64_t x, int idx)
 // Forward radix-2^R DIT network.  The twiddled operand is made canonical, so the butterfly's add
 // and subtract each need one carry fold; the roots w_16^idx = 2^(12 idx) are shift multiplies,
 // and those of idx 6 and 7 (2^72, 2^84: a product and a subtraction) are canonical already.
-template <int R, bool INV>
+// ODD_CANON: the odd inputs (the first stage's second operands) are canonical already.
+template <int R, bool ODD_CANON>
 __device__ __forceinline__ void radix_dit(uint64_t (&v)[16])
 {
-    static_assert(!INV, "the DIT network runs forward transforms");
 #pragma unroll
     for (int u = 0; u < R; u++) {
         const int h = 1 << u;
@@ -117,7 +119,7 @@ __device__ __forceinline__ void radix_dit(uint64_t (&v)[16])
             const int e = j & (h - 1);
             uint64_t x = v[j + h];
             if (e) x = mul_root16(x, e << (3 - u));
-            if ((e << (3 - u)) < 6) x = gl::canon(x);
+            if ((e << (3 - u)) < 6 && !(ODD_CANON && u == 0)) x = gl::canon(x);
             const uint64_t y = v[j];
             v[j] = gl::add_c(y, x);
             v[j + h] = gl::sub_c(y, x);
@@ -172,7 +174,7 @@ __device__ __forceinline__ void radix_phase(uint64_t *sm, uint32_t k, uint32_t l
 #pragma unroll
                 for (int j = 1; j < NR; j++) {
                     const uint32_t br = __brev((uint32_t)j) >> (32 - R);
-                    v[j] = gl::mul(v[j], __ldg(wtab + (((br * lo_m) << wsh) & 4095)));
+                    v[j] = gl::mont_mul_c(v[j], __ldg(wtab + (((br * lo_m) << wsh) & 4095)));
                 }
             }
             radix_dit<R, false>(v);
@@ -182,7 +184,7 @@ __device__ __forceinline__ void radix_phase(uint64_t *sm, uint32_t k, uint32_t l
 #pragma unroll
                 for (int j = 1; j < NR; j++) {
                     const uint32_t br = __brev((uint32_t)j) >> (32 - R);
-                    v[j] = gl::mul(v[j], __ldg(wtab + (((br * lo_m) << wsh) & 4095)));
+                    v[j] = gl::mont_mul_c(v[j], __ldg(wtab + (((br * lo_m) << wsh) & 4095)));
                 }
             }
         }
@@ -239,11 +241,11 @@ __device__ __forceinline__ void pass16_body(const Pass &a, uint64_t tile, uint64
     for (uint32_t q = threadIdx.x; q < T; q += blockDim.x) {
         const uint64_t pos = base | ((uint64_t)(q >> lgL) << s0) | (q & Lm);
         uint64_t v = S[((pos >> a.rep) << a.gshift) + a.goff];
-        if (a.scale) v = gl::mul(v, a.scale);
+        if (a.scale) v = gl::mont_mul_c(v, a.scale);
         if (!inv && s0 > 0) {
             const uint64_t lo = (lob << lgL) | (q & Lm);
             const uint64_t E = (uint64_t)brev_bits(q >> lgL, k) * lo;
-            if (E) v = gl::mul(v, big_twiddle(E << tw_shift, false));
+            if (E) v = gl::mont_mul_c(v, big_twiddle(E << tw_shift, false));
         }
         sm[pad16(q)] = v;
     }
@@ -258,13 +260,13 @@ __device__ __forceinline__ void pass16_body(const Pass &a, uint64_t tile, uint64
         if (inv && s0 > 0) {
             const uint64_t lo = (lob << lgL) | (q & Lm);
             const uint64_t E = (uint64_t)brev_bits(q >> lgL, k) * lo;
-            if (E) v = gl::mul(v, big_twiddle(E << tw_shift, true));
+            if (E) v = gl::mont_mul_c(v, big_twiddle(E << tw_shift, true));
         }
         if (a.post == POST_COSET) {
             const uint32_t br = brev_bits((uint32_t)pos, a.lg);
             const uint64_t f =
-                gl::mul(__ldg(g_ntt_sh_lo_n + (a.lg << 12) + (br & 4095)), __ldg(g_ntt_sh_hi + (br >> 12)));
-            v = gl::mul(v, f);
+                gl::mont_mul_c(__ldg(g_ntt_sh_lo_n + (a.lg << 12) + (br & 4095)), __ldg(g_ntt_sh_hi + (br >> 12)));
+            v = gl::mont_mul_c(v, f);
         } else if (a.post == POST_CANON) {
             v = gl::canon(v);
         }
@@ -322,21 +324,25 @@ __device__ __forceinline__ void radix_phase_fixed(uint64_t *sm)
 #pragma unroll
         for (int j = 0; j < NR; j++) v[j] = sm[pad_off<M>(pbase, base, j)];
         if (!DIF) {
+            // twiddled values are canonical, so the first stage takes them as they are
             if (PB && lo_m) {
 #pragma unroll
                 for (int j = 1; j < NR; j++) {
                     const uint32_t br = __brev((uint32_t)j) >> (32 - R);
-                    v[j] = gl::mul(v[j], __ldg(wtab + (((br * lo_m) << WSH) & 4095)));
+                    v[j] = gl::mont_mul_c(v[j], __ldg(wtab + (((br * lo_m) << WSH) & 4095)));
                 }
+            } else if (PB) {
+#pragma unroll
+                for (int j = 1; j < NR; j += 2) v[j] = gl::canon(v[j]);
             }
-            radix_dit<R, false>(v);
+            radix_dit<R, (PB > 0)>(v);
         } else {
             radix_dif<R, true>(v);
             if (PB && lo_m) {
 #pragma unroll
                 for (int j = 1; j < NR; j++) {
                     const uint32_t br = __brev((uint32_t)j) >> (32 - R);
-                    v[j] = gl::mul(v[j], __ldg(wtab + (((br * lo_m) << WSH) & 4095)));
+                    v[j] = gl::mont_mul_c(v[j], __ldg(wtab + (((br * lo_m) << WSH) & 4095)));
                 }
             }
         }
@@ -412,16 +418,16 @@ struct Powers {
     {
         v[0] = A;
 #pragma unroll
-        for (int c = 1; c < CH; c++) v[c] = gl::mul(v[c - 1], B);
+        for (int c = 1; c < CH; c++) v[c] = gl::mont_mul_c(v[c - 1], B);
         uint64_t s = B;
 #pragma unroll
-        for (int c = 1; c < CH; c++) s = gl::mul(s, B);  // B^CH (CH <= 4)
+        for (int c = 1; c < CH; c++) s = gl::mont_mul_c(s, B);  // B^CH (CH <= 4)
         step = s;
     }
     __device__ __forceinline__ uint64_t next(int c)
     {
         const uint64_t r = v[c];
-        v[c] = gl::mul(v[c], step);
+        v[c] = gl::mont_mul_c(v[c], step);
         return r;
     }
 };
@@ -464,7 +470,7 @@ __device__ __forceinline__ void load_tile_copies(uint64_t *sm, const uint64_t *S
             sm[pad16(mid << LGL)] = v;
 #pragma unroll
             for (int l = 1; l < (1 << LGL); l++) {
-                u = gl::mul(u, t);
+                u = gl::mont_mul_c(u, t);
                 sm[pad16((mid << LGL) | l)] = u;
             }
         }
@@ -500,8 +506,8 @@ __device__ __forceinline__ void load_tile(uint64_t *sm, const Pass &a, const uin
                 const uint32_t q = threadIdx.x + it * NT;
                 const uint32_t pos = base | ((q >> LGL) << s0) | (q & Lm);
                 uint64_t v = S[((pos >> rep) << gshift) + goff];
-                if (a.scale) v = gl::mul(v, a.scale);
-                if (tw) v = gl::mul(v, pw.next(c));
+                if (a.scale) v = gl::mont_mul_c(v, a.scale);
+                if (tw) v = gl::mont_mul_c(v, pw.next(c));
                 sm[pad16(q)] = v;
             }
         }
@@ -512,11 +518,11 @@ __device__ __forceinline__ void load_tile(uint64_t *sm, const Pass &a, const uin
             if ((T % NT) != 0 && q >= (uint32_t)T) break;
             const uint32_t pos = base | ((q >> LGL) << s0) | (q & Lm);
             uint64_t v = S[((pos >> rep) << gshift) + goff];
-            if (a.scale) v = gl::mul(v, a.scale);
+            if (a.scale) v = gl::mont_mul_c(v, a.scale);
             if (tw) {
                 const uint32_t lo = (lob << LGL) | (q & Lm);
                 const uint32_t E = (__brev(q >> LGL) >> (32 - K)) * lo;
-                if (E) v = gl::mul(v, big_twiddle((uint64_t)(E << tw_shift), false));
+                if (E) v = gl::mont_mul_c(v, big_twiddle((uint64_t)(E << tw_shift), false));
             }
             sm[pad16(q)] = v;
         }
@@ -545,9 +551,9 @@ __device__ __forceinline__ void store_tile(const uint64_t *sm, const Pass &a, ui
             const uint32_t lg = a.lg, up = lg - K;
             const uint32_t e0 = brev_bits(base, lg) + ((brev_bits(threadIdx.x, I::MB) << I::LOG_IT) << up);
             const uint64_t c0 =
-                gl::mul(__ldg(g_ntt_sh_lo_n + (lg << 12) + (e0 & 4095)), __ldg(g_ntt_sh_hi + (e0 >> 12)));
+                gl::mont_mul_c(__ldg(g_ntt_sh_lo_n + (lg << 12) + (e0 & 4095)), __ldg(g_ntt_sh_hi + (e0 >> 12)));
             const uint32_t es = 1u << up;  // 7^(2^up), without the 1/N of the lg table (lg 0: 2^0)
-            const uint64_t st = gl::mul(__ldg(g_ntt_sh_lo_n + (es & 4095)), __ldg(g_ntt_sh_hi + (es >> 12)));
+            const uint64_t st = gl::mont_mul_c(__ldg(g_ntt_sh_lo_n + (es & 4095)), __ldg(g_ntt_sh_hi + (es >> 12)));
             pw.init(c0, st);
         }
 #pragma unroll 1
@@ -559,7 +565,7 @@ __device__ __forceinline__ void store_tile(const uint64_t *sm, const Pass &a, ui
                 const uint32_t pos = base | ((q >> LGL) << s0) | (q & Lm);
                 uint64_t v = sm[pad16(q)];
                 if (tw || post == POST_COSET)
-                    v = gl::mul(v, pw.next(c));
+                    v = gl::mont_mul_c(v, pw.next(c));
                 else if (post == POST_CANON)
                     v = gl::canon(v);
                 D[pos] = v;
@@ -575,13 +581,13 @@ __device__ __forceinline__ void store_tile(const uint64_t *sm, const Pass &a, ui
             if (tw) {
                 const uint32_t lo = (lob << LGL) | (q & Lm);
                 const uint32_t E = (__brev(q >> LGL) >> (32 - K)) * lo;
-                if (E) v = gl::mul(v, big_twiddle((uint64_t)(E << tw_shift), true));
+                if (E) v = gl::mont_mul_c(v, big_twiddle((uint64_t)(E << tw_shift), true));
             }
             if (post == POST_COSET) {
                 const uint32_t br = brev_bits(pos, a.lg);
                 const uint64_t f =
-                    gl::mul(__ldg(g_ntt_sh_lo_n + (a.lg << 12) + (br & 4095)), __ldg(g_ntt_sh_hi + (br >> 12)));
-                v = gl::mul(v, f);
+                    gl::mont_mul_c(__ldg(g_ntt_sh_lo_n + (a.lg << 12) + (br & 4095)), __ldg(g_ntt_sh_hi + (br >> 12)));
+                v = gl::mont_mul_c(v, f);
             } else if (post == POST_CANON) {
                 v = gl::canon(v);
             }
@@ -975,7 +981,7 @@ inline cudaError_t lde_q(uint64_t *d_cmq, const uint64_t *d_q, bool q_rowmajor, 
         uint64_t br = 0;
         for (uint32_t t = 0; t < b; t++) br |= (uint64_t)((pc >> t) & 1) << (b - 1 - t);
         p.goff = br;
-        p.scale = glh::mul(S, next_inv);  // nonzero: a product of nonzero field elements
+        p.scale = glh::mont(glh::mul(S, next_inv));  // nonzero: a product of nonzero field elements
         p.post = (nw == 1) ? POST_CANON : POST_NONE;
         if ((err = launch_pass(p, qDim, stream)) != cudaSuccess) return err;
         S = glh::mul(S, shift_in);
@@ -1027,6 +1033,14 @@ inline cudaError_t init_tables()
             w4096_f[j] = glh::mul(w4096_f[j - 1], w4096);
             w4096_i[j] = glh::mul(w4096_i[j - 1], w4096i);
         }
+        auto to_mont = [](uint64_t *t, size_t n) {
+            for (size_t j = 0; j < n; j++) t[j] = glh::mont(t[j]);
+        };
+        for (uint64_t *t : {lo_f, hi_f, lo_i, hi_i}) to_mont(t, 1 << 13);
+        to_mont(sh_hi, 1 << 14);
+        to_mont(sh_lo_n, sizeof(sh_lo_n) / 8);
+        to_mont(w4096_f, 4096);
+        to_mont(w4096_i, 4096);
         ready = true;
     }
     cudaError_t e;
