@@ -794,8 +794,9 @@ inline void set_tuned(uint32_t nBits, uint32_t nBitsExt, uint64_t ncols, Tune t)
     tune_table()[tune_key(nBits, nBitsExt, ncols)] = t;
 }
 
-// Windows covering stages [lo, hi).  The window that starts at `lo` keeps every lower lane
-// (lgL = lo) so its tile is one contiguous run; the others take as many lanes as fill an
+// Windows covering stages [lo, hi).  The window that starts at `lo` keeps every lower lane (lgL = lo) if that fills a
+// tile, so its tile is one contiguous run, and else takes one lane (2^9 rows x 19 columns at blowup 2: 24.8 us
+// in the runtime-shaped kernel, the whole LDE 37 -> 27 us with the fixed one); the others take as many lanes as fill an
 // 8192-element tile (at most all 2^s0 of them).  kfirst / krest cap the first window and the
 // others (the autotuned plan parameters).
 inline int plan_windows(uint32_t lo, uint32_t hi, Window *w, int maxw, uint32_t kfirst = NTT_KMAX,
@@ -809,7 +810,8 @@ inline int plan_windows(uint32_t lo, uint32_t hi, Window *w, int maxw, uint32_t 
     if (k0 + lo > 13) k0 = (lo >= 13) ? 0 : 13 - lo;
     if (k0 == 0 && total > 0) return -1;  // stage offset too large for one tile
     if (krest < 1 || krest > NTT_KMAX) krest = 11;
-    w[n++] = Window{lo, k0, lo};
+    // a first window that fills no tile takes one lane of the 2^lo copies a CTA: that shape has a fixed kernel
+    w[n++] = Window{lo, k0, k0 + lo == 13 ? lo : 0};
     uint32_t rest = total - k0, s = lo + k0;
     uint32_t np = (rest + krest - 1) / krest;
     for (uint32_t i = 0; i < np; i++) {
