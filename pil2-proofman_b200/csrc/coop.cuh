@@ -167,23 +167,31 @@ __device__ __forceinline__ uint64_t permute(uint64_t x, int gbase, int k)
     const uint64_t *C = Tab<W>::C();
     const Row row = m4_row(k & 3);
     const uint64_t d = __ldg(Tab<W>::D() + kk);
+    // constants are loaded a round ahead: their latency (L2 in a fresh CTA) is as long as a round
+    auto full = [&](int r) { return __ldg(C + (r < 4 ? r * W : 4 * W + NPARTIAL + (r - 4) * W) + kk); };
+    uint64_t c = full(0);
     if (!live) x = 0;
     x = external_layer<W>(x, gbase, k, live, row);
 #pragma unroll 1
     for (int r = 0; r < 8; r++) {
-        const uint64_t c = __ldg(C + (r < 4 ? r * W : 4 * W + NPARTIAL + (r - 4) * W) + kk);
+        const uint64_t cn = full(r < 7 ? r + 1 : 0);
+        uint64_t cp = __ldg(C + 4 * W);
         x = gl::pow7(gl::add_c(x, c));
+        c = cn;
         x = external_layer<W>(x, gbase, k, live, row);
         if (r == 3) {
 #pragma unroll 1
             for (int pr = 0; pr < NPARTIAL; pr++) {
+                const uint64_t cpn = __ldg(C + 4 * W + (pr + 1 < NPARTIAL ? pr + 1 : 0));
                 // sum of x_1.. (beside the S-box of x0, which every lane computes on its own word)
                 gl::Acc rest = gl::acc((live && k != 0) ? x : 0ull);
                 rest = xor_sum<0, (G == 16 ? 4 : 3)>(rest);
-                const uint64_t s0 = gl::pow7(gl::add_c(x, __ldg(C + 4 * W + pr)));
+                const uint64_t s0 = gl::pow7(gl::add_c(x, cp));
+                cp = cpn;
                 const uint64_t x0 = shfl_u64(s0, gbase);
-                const uint64_t sum = gl::acc_reduce(gl::acc_add64(rest, x0));
-                x = gl::mul_add(k == 0 ? x0 : x, d, sum);
+                // x * d + sum in one reduction: d < p, so the product leaves 2^96 - 2^65 below 2^128
+                const unsigned __int128 v = (unsigned __int128)(k == 0 ? x0 : x) * d + (rest.v + x0);
+                x = gl::reduce128((uint32_t)v, (uint32_t)(v >> 32), (uint32_t)(v >> 64), (uint32_t)(v >> 96));
                 if (!live) x = 0;
             }
         }
@@ -265,7 +273,6 @@ __device__ __forceinline__ uint64_t permute_fam(uint64_t x, int gbase, int k)
 // Kernels.  CTAs of CTA_THREADS threads = CTA_THREADS / G states.
 // ---------------------------------------------------------------------------------
 constexpr int CTA_THREADS = 256;
-constexpr int TAIL_THREADS = 1024;
 
 // Parent i of a tree level (semantics of merkle::node_one): the W = 4 * arity child words, zero
 // past `pending`; the last parent writes the level's `pad` zero digests after its children.
@@ -282,36 +289,64 @@ __device__ __forceinline__ void node_group(uint64_t *__restrict__ level, uint64_
     if (valid && k < 4) out[i * 4 + k] = gl::canon(x);
 }
 
-template <int W, int FAM = 2>
-__global__ void __launch_bounds__(CTA_THREADS) node_coop_kernel(uint64_t *__restrict__ level, uint64_t pending,
-                                                                uint64_t pad, uint64_t parents,
-                                                                uint64_t *__restrict__ out)
-{
-    constexpr int G = Tab<W>::G;
-    const int lane = threadIdx.x & 31;
-    const uint64_t i = ((uint64_t)blockIdx.x * CTA_THREADS + threadIdx.x) / G;
-    node_group<W, FAM>(level, pending, pad, parents, out, i, lane & ~(G - 1), lane & (G - 1));
-}
+// Parents that a CTA of subtree_kernel takes on its first level: the largest power of the arity that its
+// groups hold (16 at W = 16, 9 at W = 12, 32 at W = 8), and the levels that fit above each other in it.
+template <int W>
+struct Subtree {
+    static constexpr int ARITY = W / 4, SLOTS = CTA_THREADS / Tab<W>::G;
+    static constexpr int pow_at_most(int v, int limit) { return v * ARITY > limit ? v : pow_at_most(v * ARITY, limit); }
+    static constexpr int log_of(int v) { return v < ARITY ? 0 : 1 + log_of(v / ARITY); }
+    static constexpr int PARENTS = pow_at_most(1, SLOTS), LEVELS = 1 + log_of(PARENTS);
+};
 
-// Every remaining level of a tree whose current level has `pending` digests at `level`, in one
-// CTA (the level loop runs inside; a barrier separates the levels).  Used once a level has at
-// most TAIL_THREADS / G parents.
-template <int W, int FAM = 2>
-__global__ void __launch_bounds__(TAIL_THREADS) tree_tail_kernel(uint64_t *level, uint64_t pending)
+// `levels` levels above the `pending` digests at `level`, block b's share: it takes parents [b P, b P + P) of the first level,
+// whose parents are its own too, and so on up, so a barrier of the CTA separates the levels and a small tree takes
+// a third (arity 4) or a sixth (arity 2) of the launches.  Warps without a parent skip the level: the last levels
+// of a tree in one 1024-thread CTA whose warps all ran every level took 125 us (arity 2: 229).  With the constants
+// loaded ahead and one reduction a partial round, the levels above 1024 leaves went 138 -> 50 us (arity 4) and
+// 259 -> 85 (arity 2), about 8 us a level (B200).
+template <int W, int FAM>
+__device__ __forceinline__ void subtree_block(uint64_t *level, uint64_t pending, int levels, uint64_t block)
 {
     constexpr int G = Tab<W>::G;
     constexpr uint64_t ARITY = W / 4;
     const int lane = threadIdx.x & 31;
-    const uint64_t i = threadIdx.x / G;
-    while (pending > 1) {
+    const uint64_t slot = threadIdx.x / G, first = (threadIdx.x & ~31u) / G;  // the warp's first slot
+    uint64_t n = Subtree<W>::PARENTS;
+    for (int l = 0; l < levels; l++) {
         const uint64_t pad = (ARITY - pending % ARITY) % ARITY;
         const uint64_t parents = (pending + ARITY - 1) / ARITY;
         uint64_t *out = level + (pending + pad) * 4;
-        node_group<W, FAM>(level, pending, pad, parents, out, i, lane & ~(G - 1), lane & (G - 1));
+        const uint64_t at = block * n;
+        if (first < n && at + first < parents)
+            node_group<W, FAM>(level, pending, pad, parents, out, slot < n ? at + slot : parents, lane & ~(G - 1),
+                               lane & (G - 1));
         __syncthreads();
         level = out;
         pending = parents;
+        n /= ARITY;
     }
+}
+
+template <int W, int FAM = 2>
+__global__ void __launch_bounds__(CTA_THREADS) subtree_kernel(uint64_t *level, uint64_t pending, int levels)
+{
+    subtree_block<W, FAM>(level, pending, levels, blockIdx.x);
+}
+
+// Where a launch of subtree_kernel over the `pending` digests at word `at` of a tree leaves it: moves both to the first
+// level it does not hash and returns the levels it does.
+template <int W>
+inline int subtree_advance(uint64_t &pending, uint64_t &at)
+{
+    constexpr uint64_t ARITY = W / 4;
+    int levels = 0;
+    while (pending > 1 && levels < Subtree<W>::LEVELS) {
+        at += (pending + (ARITY - pending % ARITY) % ARITY) * 4;
+        pending = (pending + ARITY - 1) / ARITY;
+        levels++;
+    }
+    return levels;
 }
 
 // Row sponge of row `row` (semantics of merkle::leaf_row): the capacity starts at zero; each block

@@ -108,13 +108,20 @@ inline uint64_t tree_num_elements(uint64_t nrows, uint64_t arity)
     return total * 4;
 }
 
-// Below this many states per launch the tiled kernels leave most of the GPU idle and take the latency of whole
-// permutations (~20 us each); the cooperative kernels (coop.cuh, one state per 16 lanes) take it instead.
-constexpr uint64_t COOP_MAX_STATES = 8192;
+// Launches of at most this many states x lanes (4096 states at W = 12 and 16, 8192 at W = 8) run cooperatively
+// (coop.cuh): below it the tiled kernels leave most of the GPU idle and take the latency of whole permutations, above
+// it the cooperative ones' instructions take longer.  One W16 permutation of 4096 / 6144 rows: 23 / 32 us cooperative,
+// 30 / 30 tiled; W8 of 8192 / 12288 rows: 21 / 30 and 23 / 23.
+constexpr uint64_t COOP_MAX_LANES = 65536;
+template <int W>
+constexpr uint64_t coop_max_states()
+{
+    return COOP_MAX_LANES / coop::Tab<W>::G;
+}
 
 // Every tree level above `nrows` leaf digests already at the start of d_tree, on `stream`.
-// Levels of more than COOP_MAX_STATES parents in 128-parent tiles, smaller ones cooperatively,
-// and the last levels (<= coop::TAIL_THREADS / G parents) in one launch; both hash families.
+// Levels of more than coop_max_states parents in 128-parent tiles, smaller ones cooperatively, several to a
+// launch (coop::subtree_kernel); both hash families.
 template <int W, int FAM = 2>
 cudaError_t build_levels(uint64_t *d_tree, uint64_t nrows, cudaStream_t stream)
 {
@@ -124,24 +131,15 @@ cudaError_t build_levels(uint64_t *d_tree, uint64_t nrows, cudaStream_t stream)
     while (pending > 1) {
         const uint64_t pad = (ARITY - pending % ARITY) % ARITY;
         const uint64_t parents = (pending + ARITY - 1) / ARITY;
+        const uint64_t before = pending;
         uint64_t *lvl = d_tree + base;
-        {
-            constexpr uint64_t G = coop::Tab<W>::G;
-            if (parents <= (uint64_t)coop::TAIL_THREADS / G) {
-                coop::tree_tail_kernel<W, FAM><<<1, coop::TAIL_THREADS, 0, stream>>>(lvl, pending);
-                prof::count();
-                break;
-            }
-            if (parents <= COOP_MAX_STATES) {
-                const uint64_t threads = parents * G;
-                coop::node_coop_kernel<W, FAM>
-                    <<<(unsigned)((threads + coop::CTA_THREADS - 1) / coop::CTA_THREADS), coop::CTA_THREADS, 0,
-                       stream>>>(lvl, pending, pad, parents, lvl + (pending + pad) * 4);
-                prof::count();
-                base += (pending + pad) * 4;
-                pending = parents;
-                continue;
-            }
+        if (parents <= coop_max_states<W>()) {
+            constexpr uint64_t P = coop::Subtree<W>::PARENTS;
+            const int levels = coop::subtree_advance<W>(pending, base);
+            coop::subtree_kernel<W, FAM><<<(unsigned)((parents + P - 1) / P), coop::CTA_THREADS, 0, stream>>>(
+                lvl, before, levels);
+            prof::count();
+            continue;
         }
         node_kernel<W, FAM><<<tch::grid((parents + 127) / 128), tch::THREADS, tch::Smem<W>::BYTES, stream>>>(
             lvl, pending, pad, parents, lvl + (pending + pad) * 4);
@@ -171,7 +169,7 @@ cudaError_t build_tree(uint64_t *d_tree, const uint64_t *d_src, uint64_t rs, uin
     if (nrows == 0) return cudaSuccess;
     {
         prof::Scope ps(prof::LEAF_HASH, stream);
-        if (nrows <= COOP_MAX_STATES) {
+        if (nrows <= coop_max_states<W>()) {
             const uint64_t threads = nrows * coop::Tab<W>::G;
             coop::leaf_coop_kernel<W, FAM><<<(unsigned)((threads + coop::CTA_THREADS - 1) / coop::CTA_THREADS),
                                              coop::CTA_THREADS, 0, stream>>>(d_tree, d_src, rs, cs, ncols, nrows);

@@ -282,7 +282,7 @@ extern "C" const char *b200_kernel_names(void)
     return "pass16_kernel\ntranspose_kernel\ntranspose_tma_kernel\nleaf_hash_kernel\nnode_kernel\npermute_kernel\nlde_rows_kernel\n"
            "fill_kernel\nimad_probe_kernel\ntranspose_grouped\npass_grouped\nleaf_persistent\n"
            "node_grouped\ngather_roots\npass_fixed_kernel\nopenings_kernel\nbitfield_unpack_kernel\n"
-           "unpack_range_kernel\npass_fixed_grouped\nnode_coop_kernel\ntree_tail_kernel\n"
+           "unpack_range_kernel\npass_fixed_grouped\nsubtree_kernel\nsubtree_grouped\n"
            "leaf_coop_kernel\n";
 }
 

@@ -1,6 +1,6 @@
 """The tensor core hashing kernels (tc_hash.cuh) against the oracle, above the cooperative kernels' range.
 
-Edges: one row into a new 128-row tile, one tile more than the resident groups (148 SMs x 4), sponges of no,
+Edges: the first row counts past that range (4096; 8192 at arity 2), one row into a new 128-row tile, one tile more than the resident groups (148 SMs x 4), sponges of no,
 one and more blocks with a full and a ragged last one, both strides, a tree at an odd word of its buffer
 (8-byte stores), words from 0 to 2^64 - 1, and a level whose last parent has missing children.
 Whole trees are compared, bit for bit.
@@ -25,7 +25,7 @@ def dev(pkg):
 
 
 # rows, columns in sponge blocks (blocks, extra columns)
-ROWS = [8193, 8320, 148 * 4 * 128 + 1]
+ROWS = [4097, 8193, 8320, 148 * 4 * 128 + 1]
 COLS = [(0, 0), (1, 0), (1, 1), (2, -1)]
 
 
@@ -55,3 +55,32 @@ def test_tree_at_the_tiles_edges(dev, arity, family, nrows):
         torch.cuda.synchronize()
         bad = np.nonzero(tree.cpu().numpy().view(np.uint64) != exp)[0]
         assert bad.size == 0, (nrows, ncols, arity, family, bad[:8])
+
+
+# Levels by subtrees of the tree (coop.cuh): one CTA's last parent and one more (16, 9, 32 parents at arity 4, 3, 2), a
+# launch's top level ending on one digest or leaving two, and missing children at every level.
+LEVELS = [(4, n) for n in (2, 4, 5, 63, 64, 65, 255, 257, 1025, 4096, 4099, 16384)] + \
+    [(3, n) for n in (2, 3, 4, 27, 28, 81, 82, 730, 6562)] + [(2, n) for n in (2, 3, 64, 65, 127, 2049, 16384, 16387)]
+
+
+@pytest.mark.parametrize("family", [1, 2])
+@pytest.mark.parametrize("arity,nrows", LEVELS)
+def test_levels_by_subtrees(dev, arity, nrows, family):
+    pkg, torch = dev
+    orc = oracle.Oracle(family=family)
+    pkg.set_native_hash_family(family)
+    digests = oracle.random_field((nrows, 4), nrows + arity)
+    digests[0] = np.uint64(oracle.P - 1)
+    tree = torch.zeros(pkg.tree_num_elements(nrows, arity), dtype=torch.int64, device="cuda")
+    tree[:4 * nrows] = torch.from_numpy(digests.reshape(-1).view(np.int64)).cuda()
+    pkg.merkletree_reduce_device(tree[:4 * nrows].clone(), nrows, arity, tree)
+    torch.cuda.synchronize()
+    got = tree.cpu().numpy().view(np.uint64)
+    level, at = digests.reshape(-1), 0
+    while level.size > 4:
+        n = level.size // 4
+        level = np.concatenate([level, np.zeros(4 * (-n % arity), np.uint64)])
+        assert (got[at:at + level.size] == level).all(), (arity, nrows, n)
+        at += level.size
+        level = np.concatenate([orc.permute(level[i:i + 4 * arity])[:4] for i in range(0, level.size, 4 * arity)])
+    assert (got[at:at + 4] == level).all()
