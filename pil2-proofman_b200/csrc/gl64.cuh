@@ -292,6 +292,17 @@ __device__ __forceinline__ uint64_t mont_mul_c(uint64_t a, uint64_t b)
     return mont_reduce<true>(r0, r1, r2, r3);
 }
 
+// -x * 2^S mod p for 32 <= S < 64, canonical: 2^96 = -1, so it is the Montgomery reduction of x << (S - 32), three
+// shifts and eight additions where the general reduction takes two products by 2^32 - 1 and a canonicalisation more.
+template <int S>
+__device__ __forceinline__ uint64_t neg_mul_pow2(uint64_t x)
+{
+    static_assert(S > 32 && S < 64, "shift out of range");
+    constexpr int T = S - 32;
+    const uint32_t x0 = lo32(x), x1 = hi32(x);
+    return mont_reduce<true>(x0 << T, __funnelshift_l(x0, x1, T), x1 >> (32 - T), 0);
+}
+
 // x^7 * 2^(-64 * 6) for x at most MONT_MAX
 __device__ __forceinline__ uint64_t mont_pow7(uint64_t x)
 {

@@ -104,8 +104,9 @@ __device__ __forceinline__ uint64_t mul_root16(uint64_t x, int idx)
 }
 
 // Forward radix-2^R DIT network.  The twiddled operand is made canonical, so the butterfly's add
-// and subtract each need one carry fold; the roots w_16^idx = 2^(12 idx) are shift multiplies,
-// and those of idx 6 and 7 (2^72, 2^84: a product and a subtraction) are canonical already.
+// and subtract each need one carry fold; the roots w_16^idx = 2^(12 idx) are shift multiplies: those of idx 6 and 7
+// (2^72, 2^84: a product and a subtraction) are canonical already, those of idx 3 to 5 (2^36 .. 2^60) come out
+// canonical and negated from a Montgomery step, so the butterfly's sum and difference change places.
 // ODD_CANON: the odd inputs (the first stage's second operands) are canonical already.
 template <int R, bool ODD_CANON>
 __device__ __forceinline__ void radix_dit(uint64_t (&v)[16])
@@ -116,11 +117,17 @@ __device__ __forceinline__ void radix_dit(uint64_t (&v)[16])
 #pragma unroll
         for (int j = 0; j < (1 << R); j++) {
             if (j & h) continue;
-            const int e = j & (h - 1);
+            const int e = j & (h - 1), idx = e << (3 - u);
             uint64_t x = v[j + h];
-            if (e) x = mul_root16(x, e << (3 - u));
-            if ((e << (3 - u)) < 6 && !(ODD_CANON && u == 0)) x = gl::canon(x);
             const uint64_t y = v[j];
+            if (idx >= 3 && idx <= 5) {
+                x = idx == 3 ? gl::neg_mul_pow2<36>(x) : idx == 4 ? gl::neg_mul_pow2<48>(x) : gl::neg_mul_pow2<60>(x);
+                v[j] = gl::sub_c(y, x);
+                v[j + h] = gl::add_c(y, x);
+                continue;
+            }
+            if (e) x = mul_root16(x, idx);
+            if (idx < 6 && !(ODD_CANON && u == 0)) x = gl::canon(x);
             v[j] = gl::add_c(y, x);
             v[j + h] = gl::sub_c(y, x);
         }
@@ -128,28 +135,36 @@ __device__ __forceinline__ void radix_dit(uint64_t (&v)[16])
 }
 
 // Inverse radix-2^R DIF network.  w_16^-idx = -2^(96 - 12 idx), so a twiddled difference is
-// (x - y) * 2^(96 - 12 idx), taken with y canonical; the untwiddled y - x with x canonical.  Either
-// way the sum and the difference need one carry fold each.
-template <int R, bool INV>
+// (x - y) * 2^(96 - 12 idx), taken with y canonical, or for the roots with a negated product (neg_mul_pow2) -(y - x) times
+// the same, with x canonical; the untwiddled y - x with x canonical.  Either way the sum and the difference need one
+// carry fold each.  Products by 2^36 and more come out canonical: `canonical` (folded at compile time, the loops
+// being unrolled) keeps the later stages from canonicalising them again.
+template <int R>
 __device__ __forceinline__ void radix_dif(uint64_t (&v)[16])
 {
-    static_assert(INV, "the DIF network runs inverse transforms");
+    bool canonical[16] = {};
 #pragma unroll
     for (int u = R - 1; u >= 0; u--) {
         const int h = 1 << u;
 #pragma unroll
         for (int j = 0; j < (1 << R); j++) {
             if (j & h) continue;
-            const int e = j & (h - 1);
-            if (e) {
-                const uint64_t y = gl::canon(v[j]), x = v[j + h];
+            const int e = j & (h - 1), idx = 8 - (e << (3 - u));
+            if (e && (idx < 3 || idx > 5)) {
+                const uint64_t y = canonical[j] ? v[j] : gl::canon(v[j]), x = v[j + h];
                 v[j] = gl::add_c(x, y);
-                v[j + h] = mul_root16(gl::sub_c(x, y), 8 - (e << (3 - u)));
+                v[j + h] = mul_root16(gl::sub_c(x, y), idx);
             } else {
-                const uint64_t y = v[j], x = gl::canon(v[j + h]);
+                const uint64_t y = v[j], x = canonical[j + h] ? v[j + h] : gl::canon(v[j + h]);
                 v[j] = gl::add_c(y, x);
-                v[j + h] = gl::sub_c(y, x);
+                const uint64_t d = gl::sub_c(y, x);
+                v[j + h] = !e         ? d
+                           : idx == 3 ? gl::neg_mul_pow2<36>(d)
+                           : idx == 4 ? gl::neg_mul_pow2<48>(d)
+                                      : gl::neg_mul_pow2<60>(d);
             }
+            canonical[j] = false;
+            canonical[j + h] = e && idx >= 3;
         }
     }
 }
@@ -179,7 +194,7 @@ __device__ __forceinline__ void radix_phase(uint64_t *sm, uint32_t k, uint32_t l
             }
             radix_dit<R, false>(v);
         } else {
-            radix_dif<R, true>(v);
+            radix_dif<R>(v);
             if (pb && lo_m) {
 #pragma unroll
                 for (int j = 1; j < NR; j++) {
@@ -290,6 +305,9 @@ template <int K, int LGL>
 struct Shape {
     static constexpr int T = 1 << (K + LGL);
     static constexpr int NT = (T / 16) < 32 ? 32 : (T / 16) > 512 ? 512 : (T / 16);
+    // Iter<K, LGL>::SPLIT: a forward window's load multiplies every element by its twiddle (s0 > 0), or its source is the
+    // inverse's last window, which stores products (s0 = 0): either way canonical
+    static constexpr bool CANON_LOAD = T % NT == 0 && NT >= (1 << LGL);
 };
 
 // padded shared-memory index of element (base + j * 2^M) for base with zero bits in
@@ -310,6 +328,7 @@ __device__ __forceinline__ void radix_phase_fixed(uint64_t *sm)
     constexpr int NT = Shape<K, LGL>::NT;
     constexpr int IT = (G + NT - 1) / NT;
     constexpr int M = PB + LGL;
+    constexpr bool CANON_IN = !DIF && PB == 0 && Shape<K, LGL>::CANON_LOAD;
     const uint64_t *wtab = DIF ? g_ntt_w4096_inv : g_ntt_w4096_fwd;
     constexpr int WSH = 12 - PB - R;  // w_{2^(PB+R)} = w_4096^(2^WSH)
 #pragma unroll
@@ -324,7 +343,8 @@ __device__ __forceinline__ void radix_phase_fixed(uint64_t *sm)
 #pragma unroll
         for (int j = 0; j < NR; j++) v[j] = sm[pad_off<M>(pbase, base, j)];
         if (!DIF) {
-            // twiddled values are canonical, so the first stage takes them as they are
+            // twiddled values are canonical, so the first stage takes them as they are: here, and in the first phase,
+            // where a SPLIT shape's load has multiplied every element (or taken the inverse's canonical ones)
             if (PB && lo_m) {
 #pragma unroll
                 for (int j = 1; j < NR; j++) {
@@ -335,9 +355,9 @@ __device__ __forceinline__ void radix_phase_fixed(uint64_t *sm)
 #pragma unroll
                 for (int j = 1; j < NR; j += 2) v[j] = gl::canon(v[j]);
             }
-            radix_dit<R, (PB > 0)>(v);
+            radix_dit<R, (PB > 0) || CANON_IN>(v);
         } else {
-            radix_dif<R, true>(v);
+            radix_dif<R>(v);
             if (PB && lo_m) {
 #pragma unroll
                 for (int j = 1; j < NR; j++) {
@@ -399,7 +419,7 @@ template <int K, int LGL>
 struct Iter {
     static constexpr int T = Shape<K, LGL>::T, NT = Shape<K, LGL>::NT, IT = (T + NT - 1) / NT;
     static constexpr int LOG_NT = log2_const(NT);
-    static constexpr bool SPLIT = (T % NT == 0) && LOG_NT >= LGL && (1 << (K + LGL)) == T;
+    static constexpr bool SPLIT = Shape<K, LGL>::CANON_LOAD;
     static constexpr int MB = SPLIT ? LOG_NT - LGL : 0;
     static constexpr int LOG_IT = SPLIT ? K - MB : 0;
     static constexpr int CH = IT < 4 ? IT : 4;  // independent product chains of the load side (latency)
