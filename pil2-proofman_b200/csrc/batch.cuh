@@ -167,13 +167,13 @@ inline cudaError_t set_grouped_fixed_attrs()
 
 // Persistent leaf sponge: the groups of every CTA claim 128-row blocks from *counter until `total` is reached.
 template <int W, int FAM>
-__global__ void __launch_bounds__(tch::THREADS, 1)
+__global__ void __launch_bounds__(tch::Cfg<W>::THREADS, 1)
     leaf_persistent(const LeafEntry *e, int n, uint64_t total, unsigned long long *counter)
 {
     extern __shared__ __align__(128) uint8_t tc_sm[];
     __shared__ tch::Shared sh;
-    __shared__ uint64_t claim[tch::GROUPS];
-    __shared__ LeafEntry entry[tch::GROUPS];  // the claimed block's instance, staged for the group
+    __shared__ uint64_t claim[tch::Cfg<W>::GROUPS];
+    __shared__ LeafEntry entry[tch::Cfg<W>::GROUPS];  // the claimed block's instance, staged for the group
     tch::Group<W, FAM> G;
     G.setup(tc_sm, sh);
     for (;;) {
@@ -193,13 +193,13 @@ __global__ void __launch_bounds__(tch::THREADS, 1)
 }
 
 template <int W, int FAM>
-__global__ void __launch_bounds__(tch::THREADS, 1) node_grouped(const NodeEntry *e, int n, uint64_t total)
+__global__ void __launch_bounds__(tch::Cfg<W>::THREADS, 1) node_grouped(const NodeEntry *e, int n, uint64_t total)
 {
     extern __shared__ __align__(128) uint8_t tc_sm[];
     __shared__ tch::Shared sh;
     tch::Group<W, FAM> G;
     G.setup(tc_sm, sh);
-    for (uint64_t b = blockIdx.x + (uint64_t)gridDim.x * G.id; b < total; b += (uint64_t)gridDim.x * tch::GROUPS) {
+    for (uint64_t b = blockIdx.x + (uint64_t)gridDim.x * G.id; b < total; b += (uint64_t)gridDim.x * tch::Cfg<W>::GROUPS) {
         const NodeEntry &E = e[find_entry(e, n, b)];
         tch::node_tile(G, E.level, E.pending, E.pad, E.parents, E.out, b - E.begin);
     }
@@ -581,13 +581,13 @@ class Plan {
                 const unsigned ctas = (unsigned)std::min<uint64_t>(L.blocks, (uint64_t)leaf_ctas);
                 const LeafEntry *le = (const LeafEntry *)ent;
                 if (family == 1) {
-                    if (L.width == 8) leaf_persistent<8, 1><<<ctas, tch::THREADS, tch::Smem<8>::BYTES, s>>>(le, L.n, L.blocks, ctr + L.smem);
-                    if (L.width == 12) leaf_persistent<12, 1><<<ctas, tch::THREADS, tch::Smem<12>::BYTES, s>>>(le, L.n, L.blocks, ctr + L.smem);
-                    if (L.width == 16) leaf_persistent<16, 1><<<ctas, tch::THREADS, tch::Smem<16>::BYTES, s>>>(le, L.n, L.blocks, ctr + L.smem);
+                    if (L.width == 8) leaf_persistent<8, 1><<<ctas, tch::Cfg<8>::THREADS, tch::Smem<8>::BYTES, s>>>(le, L.n, L.blocks, ctr + L.smem);
+                    if (L.width == 12) leaf_persistent<12, 1><<<ctas, tch::Cfg<12>::THREADS, tch::Smem<12>::BYTES, s>>>(le, L.n, L.blocks, ctr + L.smem);
+                    if (L.width == 16) leaf_persistent<16, 1><<<ctas, tch::Cfg<16>::THREADS, tch::Smem<16>::BYTES, s>>>(le, L.n, L.blocks, ctr + L.smem);
                 } else {
-                    if (L.width == 8) leaf_persistent<8, 2><<<ctas, tch::THREADS, tch::Smem<8>::BYTES, s>>>(le, L.n, L.blocks, ctr + L.smem);
-                    if (L.width == 12) leaf_persistent<12, 2><<<ctas, tch::THREADS, tch::Smem<12>::BYTES, s>>>(le, L.n, L.blocks, ctr + L.smem);
-                    if (L.width == 16) leaf_persistent<16, 2><<<ctas, tch::THREADS, tch::Smem<16>::BYTES, s>>>(le, L.n, L.blocks, ctr + L.smem);
+                    if (L.width == 8) leaf_persistent<8, 2><<<ctas, tch::Cfg<8>::THREADS, tch::Smem<8>::BYTES, s>>>(le, L.n, L.blocks, ctr + L.smem);
+                    if (L.width == 12) leaf_persistent<12, 2><<<ctas, tch::Cfg<12>::THREADS, tch::Smem<12>::BYTES, s>>>(le, L.n, L.blocks, ctr + L.smem);
+                    if (L.width == 16) leaf_persistent<16, 2><<<ctas, tch::Cfg<16>::THREADS, tch::Smem<16>::BYTES, s>>>(le, L.n, L.blocks, ctr + L.smem);
                 }
                 break;
             }
@@ -608,13 +608,13 @@ class Plan {
                 const unsigned ctas = (unsigned)std::min<uint64_t>(L.blocks, (uint64_t)leaf_ctas);
                 const NodeEntry *ne = (const NodeEntry *)ent;
                 if (family == 1) {
-                    if (L.width == 8) node_grouped<8, 1><<<ctas, tch::THREADS, tch::Smem<8>::BYTES, s>>>(ne, L.n, L.blocks);
-                    if (L.width == 12) node_grouped<12, 1><<<ctas, tch::THREADS, tch::Smem<12>::BYTES, s>>>(ne, L.n, L.blocks);
-                    if (L.width == 16) node_grouped<16, 1><<<ctas, tch::THREADS, tch::Smem<16>::BYTES, s>>>(ne, L.n, L.blocks);
+                    if (L.width == 8) node_grouped<8, 1><<<ctas, tch::Cfg<8>::THREADS, tch::Smem<8>::BYTES, s>>>(ne, L.n, L.blocks);
+                    if (L.width == 12) node_grouped<12, 1><<<ctas, tch::Cfg<12>::THREADS, tch::Smem<12>::BYTES, s>>>(ne, L.n, L.blocks);
+                    if (L.width == 16) node_grouped<16, 1><<<ctas, tch::Cfg<16>::THREADS, tch::Smem<16>::BYTES, s>>>(ne, L.n, L.blocks);
                 } else {
-                    if (L.width == 8) node_grouped<8, 2><<<ctas, tch::THREADS, tch::Smem<8>::BYTES, s>>>(ne, L.n, L.blocks);
-                    if (L.width == 12) node_grouped<12, 2><<<ctas, tch::THREADS, tch::Smem<12>::BYTES, s>>>(ne, L.n, L.blocks);
-                    if (L.width == 16) node_grouped<16, 2><<<ctas, tch::THREADS, tch::Smem<16>::BYTES, s>>>(ne, L.n, L.blocks);
+                    if (L.width == 8) node_grouped<8, 2><<<ctas, tch::Cfg<8>::THREADS, tch::Smem<8>::BYTES, s>>>(ne, L.n, L.blocks);
+                    if (L.width == 12) node_grouped<12, 2><<<ctas, tch::Cfg<12>::THREADS, tch::Smem<12>::BYTES, s>>>(ne, L.n, L.blocks);
+                    if (L.width == 16) node_grouped<16, 2><<<ctas, tch::Cfg<16>::THREADS, tch::Smem<16>::BYTES, s>>>(ne, L.n, L.blocks);
                 }
                 break;
             }

@@ -49,9 +49,9 @@ __device__ __forceinline__ void permute_fam(uint64_t *st)
 // Row sponges of `nrows` rows, 128-row tiles over the groups of every CTA (tc_hash.cuh), tile t to CTA t mod the
 // grid first so that few tiles spread over the SMs.  Against one thread a row with the state in shared memory and
 // every layer on the integer pipes, 2^20 rows (B200): Poseidon2 W16 x 256 columns 24.6 -> 16.4 ms (937 -> 1403 M
-// permutations/s), W12 x 128 13.9 -> 9.8, W8 x 64 9.6 -> 7.5; Poseidon1 W16 39.0 -> 16.3, W12 19.4 -> 9.7, W8 12.5 -> 7.4.
+// permutations/s), W12 x 128 13.9 -> 9.8, W8 x 64 9.6 -> 7.0; Poseidon1 W16 39.0 -> 16.4, W12 19.4 -> 9.7, W8 12.5 -> 7.0.
 template <int W, int FAM = 2>
-__global__ void __launch_bounds__(tch::THREADS, 1) leaf_hash_kernel(uint64_t *__restrict__ digests,
+__global__ void __launch_bounds__(tch::Cfg<W>::THREADS, 1) leaf_hash_kernel(uint64_t *__restrict__ digests,
                                                                     const uint64_t *__restrict__ src, uint64_t rs,
                                                                     uint64_t cs, uint64_t ncols, uint64_t nrows,
                                                                     int resume)
@@ -61,14 +61,14 @@ __global__ void __launch_bounds__(tch::THREADS, 1) leaf_hash_kernel(uint64_t *__
     tch::Group<W, FAM> G;
     G.setup(tc_sm, sh);
     const uint64_t tiles = (nrows + 127) / 128;
-    for (uint64_t t = blockIdx.x + (uint64_t)gridDim.x * G.id; t < tiles; t += (uint64_t)gridDim.x * tch::GROUPS)
+    for (uint64_t t = blockIdx.x + (uint64_t)gridDim.x * G.id; t < tiles; t += (uint64_t)gridDim.x * tch::Cfg<W>::GROUPS)
         tch::leaf_tile(G, digests, src, rs, cs, ncols, nrows, t, resume != 0);
     G.finish(sh);
 }
 
 // One tree level of `parents` parents.
 template <int W, int FAM = 2>
-__global__ void __launch_bounds__(tch::THREADS, 1) node_kernel(uint64_t *__restrict__ level, uint64_t pending, uint64_t pad,
+__global__ void __launch_bounds__(tch::Cfg<W>::THREADS, 1) node_kernel(uint64_t *__restrict__ level, uint64_t pending, uint64_t pad,
                                                                uint64_t parents, uint64_t *__restrict__ out)
 {
     extern __shared__ __align__(128) uint8_t tc_sm[];
@@ -76,7 +76,7 @@ __global__ void __launch_bounds__(tch::THREADS, 1) node_kernel(uint64_t *__restr
     tch::Group<W, FAM> G;
     G.setup(tc_sm, sh);
     const uint64_t tiles = (parents + 127) / 128;
-    for (uint64_t t = blockIdx.x + (uint64_t)gridDim.x * G.id; t < tiles; t += (uint64_t)gridDim.x * tch::GROUPS)
+    for (uint64_t t = blockIdx.x + (uint64_t)gridDim.x * G.id; t < tiles; t += (uint64_t)gridDim.x * tch::Cfg<W>::GROUPS)
         tch::node_tile(G, level, pending, pad, parents, out, t);
     G.finish(sh);
 }
@@ -111,7 +111,7 @@ inline uint64_t tree_num_elements(uint64_t nrows, uint64_t arity)
 // Launches of at most this many states x lanes (4096 states at W = 12 and 16, 8192 at W = 8) run cooperatively
 // (coop.cuh): below it the tiled kernels leave most of the GPU idle and take the latency of whole permutations, above
 // it the cooperative ones' instructions take longer.  One W16 permutation of 4096 / 6144 rows: 23 / 32 us cooperative,
-// 30 / 30 tiled; W8 of 8192 / 12288 rows: 21 / 30 and 23 / 23.
+// 30 / 30 tiled; W8 of 8192 / 12288 rows: 21 / 30 and 26 / 26.
 constexpr uint64_t COOP_MAX_LANES = 65536;
 template <int W>
 constexpr uint64_t coop_max_states()
@@ -141,7 +141,7 @@ cudaError_t build_levels(uint64_t *d_tree, uint64_t nrows, cudaStream_t stream)
             prof::count();
             continue;
         }
-        node_kernel<W, FAM><<<tch::grid((parents + 127) / 128), tch::THREADS, tch::Smem<W>::BYTES, stream>>>(
+        node_kernel<W, FAM><<<tch::grid((parents + 127) / 128), tch::Cfg<W>::THREADS, tch::Smem<W>::BYTES, stream>>>(
             lvl, pending, pad, parents, lvl + (pending + pad) * 4);
         prof::count();
         base += (pending + pad) * 4;
@@ -155,7 +155,7 @@ template <int W, int FAM = 2>
 cudaError_t hash_rows(uint64_t *digests, const uint64_t *src, uint64_t rs, uint64_t cs, uint64_t ncols, uint64_t nrows,
                       bool resume, cudaStream_t stream)
 {
-    leaf_hash_kernel<W, FAM><<<tch::grid((nrows + 127) / 128), tch::THREADS, tch::Smem<W>::BYTES, stream>>>(
+    leaf_hash_kernel<W, FAM><<<tch::grid((nrows + 127) / 128), tch::Cfg<W>::THREADS, tch::Smem<W>::BYTES, stream>>>(
         digests, src, rs, cs, ncols, nrows, resume ? 1 : 0);
     prof::count();
     return cudaGetLastError();

@@ -13,10 +13,11 @@
 // joining eight columns costs a third of the 128-bit sums that it replaces.  The S-boxes and joins run in
 // Montgomery form because that reduction needs no multiplication (gl64.cuh).
 //
-// A CTA is four groups, one CTA an SM: the tables take 106 KB of shared memory at width 16, each group 28 KB and a
+// At width 12 and 16 a CTA is four groups, one CTA an SM: the tables take 106 KB of shared memory at width 16, each group 28 KB and a
 // quarter of the tensor memory (128 columns, a whole layer's).  Two threads share a row (each takes half its words, and
 // every other run of partial rounds), so 32 warps hide the barriers and latencies: one row of 128 rows x 40 columns
-// takes 20 % less than with one thread a row, large launches the same.  Groups run independently, so one's products
+// takes 20 % less than with one thread a row, large launches the same.  At width 8 a layer has 64 columns and
+// the tables 44 KB, so eight groups fit with one thread a row: 2^20 rows x 64 columns 7.5 -> 7.0 ms.  Groups run independently, so one's products
 // and barriers run under the others' S-boxes.
 #pragma once
 #include "gl64.cuh"
@@ -30,14 +31,22 @@ __constant__ tch::Consts c_tc[2][3];
 
 namespace tch {
 
-constexpr int GROUPS = 4, SPLIT = 2, STEP = 2, GTHREADS = 128 * SPLIT, THREADS = GTHREADS * GROUPS;
-constexpr uint32_t GROUP_COLS = 512 / GROUPS;  // tensor memory columns of a group
-constexpr uint32_t WAIT_LIMIT = 1u << 20;      // try_wait rounds before a thread gives up
+// Groups of a CTA, threads that share a row, and a group's tensor memory columns (a whole layer's): what shared
+// memory and the 512 columns hold, with 1024 threads either way.  (Width 12 with five groups of one thread a row: 9.65 against
+// 9.75 ms for 2^20 rows x 128 columns, but 32 against 28 us for 5000 rows x 8.)
+template <int W>
+struct Cfg {
+    static constexpr int GROUPS = W == 8 ? 8 : 4, SPLIT = W == 8 ? 1 : 2;
+    static constexpr int GTHREADS = 128 * SPLIT, THREADS = GTHREADS * GROUPS, COLS = 8 * W;
+    static_assert(GROUPS * COLS <= 512 && GROUPS <= 15, "tensor memory columns, barriers");
+};
+constexpr int MAX_GROUPS = 8;
+constexpr uint32_t WAIT_LIMIT = 1u << 20;  // try_wait rounds before a thread gives up
 
 template <int W>
 struct Smem {
     static constexpr int GROUP = (Shape<W>::CHX + YCH) * 2048;  // state rows and a block's y rows
-    static constexpr int BYTES = Shape<W>::BYTES + GROUPS * GROUP;
+    static constexpr int BYTES = Shape<W>::BYTES + Cfg<W>::GROUPS * GROUP;
 };
 
 __device__ __forceinline__ uint32_t smem_addr(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -83,7 +92,7 @@ struct Wide {
     uint32_t w[5];
 };
 
-// Column pairs: t_i = col[2i] + 256 col[2i+1] < 2^31 (check_bounds), the word is sum_i t_i 2^(16 i).
+// Column pairs: t_i = col[2i] + 256 col[2i+1], below 2^31 for every table, the word is sum_i t_i 2^(16 i).
 __device__ __forceinline__ void pairs(const uint32_t *col, uint32_t (&t)[4])
 {
 #pragma unroll
@@ -144,22 +153,27 @@ __device__ __forceinline__ uint64_t wide_reduce(const Wide &a)
     return gl::sub_c(gl::reduce128(a.w[0], a.w[1], a.w[2], a.w[3]), (uint64_t)a.w[4] << 32);
 }
 
-// Two canonical words to p: one 16-byte store where p is aligned for it (a tree may start at any word of a
-// caller's buffer), else two 8-byte ones.
-__device__ __forceinline__ void store_pair(uint64_t *p, const uint64_t (&v)[2])
+// Canonical words to p: 16-byte stores where p is aligned for them (a tree may start at any word of a caller's
+// buffer), else 8-byte ones.
+template <int N>
+__device__ __forceinline__ void store_words(uint64_t *p, const uint64_t (&v)[N])
 {
-    const uint64_t a = gl::canon(v[0]), b = gl::canon(v[1]);
-    if ((reinterpret_cast<uintptr_t>(p) & 15) == 0) {
-        *reinterpret_cast<ulonglong2 *>(p) = make_ulonglong2(a, b);
-    } else {
-        p[0] = a;
-        p[1] = b;
+    const bool aligned = (reinterpret_cast<uintptr_t>(p) & 15) == 0;
+#pragma unroll
+    for (int i = 0; i < N; i += 2) {
+        const uint64_t a = gl::canon(v[i]), b = gl::canon(v[i + 1]);
+        if (aligned) {
+            *reinterpret_cast<ulonglong2 *>(p + i) = make_ulonglong2(a, b);
+        } else {
+            p[i] = a;
+            p[i + 1] = b;
+        }
     }
 }
 
 // A CTA's barriers and tensor memory address.
 struct Shared {
-    uint64_t mbar[GROUPS];
+    uint64_t mbar[MAX_GROUPS];
     uint32_t tmem;
 };
 
@@ -175,6 +189,8 @@ struct Group {
     uint32_t half;     // this thread's share of the row's words
     bool issuer, dead;
 
+    static constexpr int GROUPS = Cfg<W>::GROUPS, SPLIT = Cfg<W>::SPLIT, GTHREADS = Cfg<W>::GTHREADS,
+                         THREADS = Cfg<W>::THREADS;
     static constexpr int OUT = 4 / SPLIT;  // output words of a thread
 
     static __device__ __forceinline__ const Consts &consts() { return c_tc[FAM - 1][W / 4 - 2]; }
@@ -201,14 +217,14 @@ struct Group {
         __syncthreads();
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         id = threadIdx.x / GTHREADS;
-        half = (threadIdx.x >> 7) & (SPLIT - 1);
+        half = (threadIdx.x >> 7) % SPLIT;
         const uint32_t r = threadIdx.x & 127;
         tab = smem_addr(sm);
         row = tab + Shape<W>::BYTES + id * Smem<W>::GROUP + r * 16;
-        tmem = sh.tmem + id * GROUP_COLS + ((warp & 3) << 21);
+        tmem = sh.tmem + id * Cfg<W>::COLS + ((warp & 3) << 21);
         mbar = smem_addr(sh.mbar + id);
         phase = 0;
-        issuer = (threadIdx.x & (GTHREADS - 1)) == 0;
+        issuer = threadIdx.x % GTHREADS == 0;
         dead = false;
     }
 
@@ -315,26 +331,29 @@ struct Group {
             }
             const uint64_t *k = C.lay[s];
 #pragma unroll 1
-            for (int i = 0; i < W / SPLIT; i += STEP) {
+            for (int i = 0; i < W / SPLIT; i += 2) {
                 const int g = half * (W / SPLIT) + i;
-                uint32_t col[8 * STEP];
+                uint32_t col[16];
                 ld_cols16(col, tmem + 8 * g);
-                uint64_t x[STEP];
+                uint64_t x[2];
 #pragma unroll
-                for (int j = 0; j < STEP; j++) x[j] = join_word(col + 8 * j, k[g + j]);
+                for (int j = 0; j < 2; j++) x[j] = join_word(col + 8 * j, k[g + j]);
                 if (s != 4) {
 #pragma unroll
-                    for (int j = 0; j < STEP; j++) x[j] = gl::mont_pow7(x[j]);
+                    for (int j = 0; j < 2; j++) x[j] = gl::mont_pow7(x[j]);
                 }
 #pragma unroll
-                for (int j = 0; j < STEP; j += 2) sts128(word_addr(g + j), x[j], x[j + 1]);
+                for (int j = 0; j < 2; j += 2) sts128(word_addr(g + j), x[j], x[j + 1]);
             }
         }
         product(S::OFF_F, S::KX / 32, S::NF, instr_desc(S::NF));
-        uint32_t col[8 * OUT];
-        ld_cols16(col, tmem + 8 * OUT * half);
 #pragma unroll
-        for (int j = 0; j < OUT; j++) out[j] = join_word(col + 8 * j, 0);
+        for (int j = 0; j < OUT; j += 2) {
+            uint32_t col[16];
+            ld_cols16(col, tmem + 8 * (OUT * half + j));
+            out[j] = join_word(col, 0);
+            out[j + 1] = join_word(col + 8, 0);
+        }
     }
 
     // words g and g + 1 of a state into the rows (g even)
@@ -358,7 +377,7 @@ __device__ __forceinline__ void leaf_tile(Group<W, FAM> &G, uint64_t *__restrict
                                           const uint64_t *__restrict__ src, uint64_t rs, uint64_t cs, uint64_t ncols,
                                           uint64_t nrows, uint64_t tile, bool resume)
 {
-    constexpr int RATE = W - 4, MINE = RATE / SPLIT, OUT = Group<W, FAM>::OUT;
+    constexpr int RATE = W - 4, MINE = RATE / Cfg<W>::SPLIT, OUT = Group<W, FAM>::OUT;
     uint64_t row = tile * 128 + (threadIdx.x & 127);
     const bool valid = row < nrows;
     if (!valid) row = nrows - 1;
@@ -377,10 +396,11 @@ __device__ __forceinline__ void leaf_tile(Group<W, FAM> &G, uint64_t *__restrict
         for (int i = 0; i < MINE; i++) v[i] = at + i < ncols ? __ldg(p + (at + i) * cs) : 0ull;
 #pragma unroll
         for (int i = 0; i < MINE; i += 2) G.put2(first + i, v[i], v[i + 1]);
-        G.put2(RATE + (int)G.half * OUT, cap[0], cap[1]);
+#pragma unroll
+        for (int i = 0; i < OUT; i += 2) G.put2(RATE + (int)G.half * OUT + i, cap[i], cap[i + 1]);
         G.permute(cap);
     }
-    if (valid) store_pair(d, cap);
+    if (valid) store_words(d, cap);
 }
 
 // Parents of up to 128 nodes of one tree level (poseidon2_goldilocks.cpp:129-175): `pending` child digests at
@@ -390,7 +410,7 @@ template <int W, int FAM>
 __device__ __forceinline__ void node_tile(Group<W, FAM> &G, uint64_t *__restrict__ level, uint64_t pending, uint64_t pad,
                                           uint64_t parents, uint64_t *__restrict__ out, uint64_t tile)
 {
-    constexpr int MINE = W / SPLIT;
+    constexpr int MINE = W / Cfg<W>::SPLIT, OUT = Group<W, FAM>::OUT;
     const uint64_t i = tile * 128 + (threadIdx.x & 127);
     const uint64_t first = i * W + G.half * MINE, end = pending * 4;
     if (i == parents - 1 && G.half == 0)
@@ -410,9 +430,9 @@ __device__ __forceinline__ void node_tile(Group<W, FAM> &G, uint64_t *__restrict
     }
 #pragma unroll
     for (int j = 0; j < MINE; j += 2) G.put2((int)G.half * MINE + j, v[j], v[j + 1]);
-    uint64_t o[2];
+    uint64_t o[OUT];
     G.permute(o);
-    if (i < parents) store_pair(out + i * 4 + G.half * 2, o);
+    if (i < parents) store_words(out + i * 4 + G.half * OUT, o);
 }
 
 // ------------------------------------------------------------------ host side ----
