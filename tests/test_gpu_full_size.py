@@ -99,8 +99,8 @@ def test_full_size_matches_reference_cpu(dev, fx):
     seeded trace (NTT_Goldilocks::LDE + Poseidon2Goldilocks<16>::merkletree, or
     PoseidonGoldilocks<16>::merkletree for the family-1 record, run by
     make_full_size.py): the one-pass device commit (root, the whole tree buffer by SHA-256, sampled
-    LDE rows word for word), then commit_witness from pinned host memory (column blocks of 16
-    columns, growing to 64, crossing PCIe while earlier blocks are extended; the sponge absorbed in 12-column
+    LDE rows word for word), then commit_witness from pinned host memory (column blocks of 16, 24,
+    48, then 64, crossing PCIe while earlier blocks are extended; the sponge absorbed in 12-column
     chunks on the idle device) to the same root."""
     pkg, torch = dev
     nbits, nbe, ncols, arity = fx["nBits"], fx["nBitsExt"], fx["nCols"], fx["arity"]
