@@ -55,6 +55,9 @@ static int ensure_init_current()
        "pass16_kernel smem attribute");
     CK(ntt::set_fixed_attrs(), "pass_fixed_kernel smem attributes");
     CK(merkle::init(), "hash tables");
+    // A copy from pageable memory may return once its source is staged, before the device has it, and callers' streams
+    // (non-blocking ones among them) are not ordered after the legacy stream that the table copies are on.
+    CK(cudaStreamSynchronize(cudaStreamLegacy), "table upload");
     g_init_done[dev] = true;
     return B200_OK;
 }
