@@ -545,7 +545,10 @@ class Plan {
         if (d_table) return cudaSuccess;
         cudaError_t e = cudaMalloc((void **)&d_table, table.size());
         if (e != cudaSuccess) return e;
+        // waited for: a copy from pageable memory may return before the device has it, and run()'s stream need not be
+        // ordered after the legacy one
         e = cudaMemcpy(d_table, table.data(), table.size(), cudaMemcpyHostToDevice);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(cudaStreamLegacy);
         if (e != cudaSuccess) return e;
         return cudaMallocHost((void **)&h_roots, 32 * (inst.size() + 1));
     }

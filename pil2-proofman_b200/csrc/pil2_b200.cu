@@ -1577,8 +1577,10 @@ extern "C" void register_instruction_table(void *d_buffers, uint64_t airgroupId,
     if (a.d_table) cudaFree(a.d_table);
     a.d_table = nullptr;
     const uint64_t words = num_entries * (words_per_entry ? words_per_entry : 1);
+    // the copy is waited for: the slots' streams are not ordered after the legacy stream
     if (cudaMalloc((void **)&a.d_table, words * 8) != cudaSuccess ||
-        cudaMemcpy(a.d_table, table, num_entries * words_per_entry * 8, cudaMemcpyHostToDevice) != cudaSuccess) {
+        cudaMemcpy(a.d_table, table, num_entries * words_per_entry * 8, cudaMemcpyHostToDevice) != cudaSuccess ||
+        cudaStreamSynchronize(cudaStreamLegacy) != cudaSuccess) {
         cudaGetLastError();
         if (a.d_table) cudaFree(a.d_table);
         a.d_table = nullptr;
