@@ -331,13 +331,18 @@ uint64_t b200_launch_count(void);
  * Accelerator where the source is 16-byte aligned with an even column count, 0 always uses the
  * thread-loaded shared-memory tiles.  Same values either way; returns the previous setting. */
 int b200_set_transpose_tma(int on);
-/* 1 if a TMA transpose tile copy did not land within the kernel's wait bound since the last call
- * (the flag is then reset), 0 otherwise, < 0 on a CUDA error. */
+/* 1 if a bounded wait ran out on the current device since the last call (a TMA transpose's tile copy or a
+ * tensor core product of the hashing kernels; the flag is then reset), 0 otherwise, < 0 on a CUDA error. */
 int b200_tma_wait_errors(void);
 
 /* INT32 multiply-add throughput probe: `blocks` x 256 threads each run 8 independent
  * mad.lo/mad.hi chains of `iters` steps; returns the measured rate in G IMAD/s. */
 int b200_probe_imad(uint64_t blocks, uint64_t iters, double *gimad_per_s);
+
+/* What the hashing kernels do when a tensor core product does not complete: one CTA runs `before` products, waits
+ * a few rounds for one that is never issued, and calls `after` more.  counts3: threads that gave up, threads that
+ * saw the missing product land, threads told to leave.  Raises the flag above. */
+int b200_probe_product_wait(uint32_t before, uint32_t after, uint32_t *counts3);
 
 /* ---- FRI query openings from the resident LDE and tree ----
  * One opening = MerkleTreeGL::getGroupProof (merkleTreeGL.cpp:145-175): the row's nCols values,

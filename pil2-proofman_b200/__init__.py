@@ -85,6 +85,7 @@ _SIGS = {
     "b200_set_transpose_tma": (_i32, [_i32]),
     "b200_tma_wait_errors": (_i32, []),
     "b200_probe_imad": (_i32, [_u64, _u64, ctypes.POINTER(ctypes.c_double)]),
+    "b200_probe_product_wait": (_i32, [ctypes.c_uint32, ctypes.c_uint32, _vp]),
     "b200_batch_plan_new": (_vp, [_vp, _u64]),
     "b200_batch_plan_run": (_i32, [_vp, _vp, _vp, _i32]),
     "b200_batch_plan_free": (None, [_vp]),

@@ -187,7 +187,7 @@ __global__ void __launch_bounds__(tch::Cfg<W>::THREADS, 1)
         if (b >= total) break;
         const LeafEntry &L = entry[G.id];
         tch::leaf_tile(G, L.digests, L.src, 1, L.nrows, L.ncols, L.nrows, b - L.begin, false);
-        G.sync();
+        if (G.gave_up()) break;
     }
     G.finish(sh);
 }
@@ -202,6 +202,7 @@ __global__ void __launch_bounds__(tch::Cfg<W>::THREADS, 1) node_grouped(const No
     for (uint64_t b = blockIdx.x + (uint64_t)gridDim.x * G.id; b < total; b += (uint64_t)gridDim.x * tch::Cfg<W>::GROUPS) {
         const NodeEntry &E = e[find_entry(e, n, b)];
         tch::node_tile(G, E.level, E.pending, E.pad, E.parents, E.out, b - E.begin);
+        if (G.gave_up()) break;
     }
     G.finish(sh);
 }

@@ -61,8 +61,10 @@ __global__ void __launch_bounds__(tch::Cfg<W>::THREADS, 1) leaf_hash_kernel(uint
     tch::Group<W, FAM> G;
     G.setup(tc_sm, sh);
     const uint64_t tiles = (nrows + 127) / 128;
-    for (uint64_t t = blockIdx.x + (uint64_t)gridDim.x * G.id; t < tiles; t += (uint64_t)gridDim.x * tch::Cfg<W>::GROUPS)
+    for (uint64_t t = blockIdx.x + (uint64_t)gridDim.x * G.id; t < tiles; t += (uint64_t)gridDim.x * tch::Cfg<W>::GROUPS) {
         tch::leaf_tile(G, digests, src, rs, cs, ncols, nrows, t, resume != 0);
+        if (G.gave_up()) break;
+    }
     G.finish(sh);
 }
 
@@ -76,8 +78,10 @@ __global__ void __launch_bounds__(tch::Cfg<W>::THREADS, 1) node_kernel(uint64_t 
     tch::Group<W, FAM> G;
     G.setup(tc_sm, sh);
     const uint64_t tiles = (parents + 127) / 128;
-    for (uint64_t t = blockIdx.x + (uint64_t)gridDim.x * G.id; t < tiles; t += (uint64_t)gridDim.x * tch::Cfg<W>::GROUPS)
+    for (uint64_t t = blockIdx.x + (uint64_t)gridDim.x * G.id; t < tiles; t += (uint64_t)gridDim.x * tch::Cfg<W>::GROUPS) {
         tch::node_tile(G, level, pending, pad, parents, out, t);
+        if (G.gave_up()) break;
+    }
     G.finish(sh);
 }
 
@@ -221,6 +225,9 @@ inline cudaError_t init()
     if (e == cudaSuccess) e = set_attrs<12, 2>();
     if (e == cudaSuccess) e = set_attrs<16, 1>();
     if (e == cudaSuccess) e = set_attrs<16, 2>();
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(tch::product_wait_probe_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 tch::Smem<16>::BYTES);
     return e;
 }
 

@@ -286,7 +286,7 @@ extern "C" const char *b200_kernel_names(void)
            "fill_kernel\nimad_probe_kernel\ntranspose_grouped\npass_grouped\nleaf_persistent\n"
            "node_grouped\ngather_roots\npass_fixed_kernel\nopenings_kernel\nbitfield_unpack_kernel\n"
            "unpack_range_kernel\npass_fixed_grouped\nsubtree_kernel\nsubtree_grouped\n"
-           "leaf_coop_kernel\n";
+           "leaf_coop_kernel\nproduct_wait_probe_kernel\n";
 }
 
 // ------------------------------------------------------------ host-buffer API ----
@@ -1098,6 +1098,19 @@ extern "C" int b200_probe_imad(uint64_t blocks, uint64_t iters, double *gimad_pe
     return B200_OK;
 }
 
+extern "C" int b200_probe_product_wait(uint32_t before, uint32_t after, uint32_t *counts3)
+{
+    int rc = ensure_init_current();
+    if (rc) return rc;
+    if (before > 64 || after > 64 || !counts3) return set_err(B200_EINVAL, "probe: at most 64 products, counts non-null");
+    DevBuf out;
+    if (out.alloc(2)) return set_err(B200_ENOMEM, "cudaMalloc");
+    CK(cudaMemset(out.p, 0, 16), "probe counts");
+    tch::product_wait_probe_kernel<<<1, tch::Cfg<16>::THREADS, tch::Smem<16>::BYTES>>>(before, after, (uint32_t *)out.p);
+    CK(cudaGetLastError(), "probe");
+    CK(cudaMemcpy(counts3, out.p, 12, cudaMemcpyDeviceToHost), "probe");
+    return B200_OK;
+}
 
 // ---------------------------------------------------- batched commit and server ----
 #include "batch_api.cuh"

@@ -195,7 +195,11 @@ struct Group {
 
     static __device__ __forceinline__ const Consts &consts() { return c_tc[FAM - 1][W / 4 - 2]; }
 
-    __device__ __forceinline__ uint32_t word_addr(int i) const { return row + (uint32_t)(i >> 1) * 2048 + (i & 1) * 8; }
+    // words i and i + 1 (i even) of this thread's row
+    __device__ __forceinline__ void store_row(int i, uint64_t x, uint64_t y) const
+    {
+        sts128(row + (uint32_t)(i >> 1) * 2048, x, y);
+    }
 
     // Tables into shared memory, tensor memory, barriers.  All threads of the CTA.
     __device__ __forceinline__ void setup(uint8_t *sm, Shared &sh)
@@ -231,16 +235,30 @@ struct Group {
     // barrier of the group's threads
     __device__ __forceinline__ void sync() const { asm volatile("bar.sync %0, %1;" ::"r"(id + 1), "n"(GTHREADS) : "memory"); }
 
-    __device__ __forceinline__ bool wait(uint32_t parity)
+    // the same barrier, and whether any of them has given up: the same answer to all, so that they leave a loop together
+    __device__ __forceinline__ bool gave_up() const
     {
-        for (uint32_t i = 0; i < WAIT_LIMIT; i++) {
+        uint32_t any;
+        asm volatile(
+            "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\t"
+            "bar.red.or.pred q, %2, %3, p;\n\t"
+            "selp.u32 %0, 1, 0, q;\n\t}"
+            : "=r"(any)
+            : "r"((uint32_t)dead), "r"(id + 1), "n"(GTHREADS)
+            : "memory");
+        return any != 0;
+    }
+
+    __device__ __forceinline__ bool wait(uint32_t limit = WAIT_LIMIT) const
+    {
+        for (uint32_t i = 0; i < limit; i++) {
             uint32_t done;
             asm volatile(
                 "{\n\t.reg .pred p;\n\t"
                 "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
                 "selp.u32 %0, 1, 0, p;\n\t}"
                 : "=r"(done)
-                : "r"(mbar), "r"(parity)
+                : "r"(mbar), "r"(phase)
                 : "memory");
             if (done) return true;
         }
@@ -249,13 +267,18 @@ struct Group {
 
     // The group's rows times a table of K bytes (K / 32 steps of 32) whose pieces hold `ld` columns, the first
     // n of them into the group's tensor memory.  Ends with the columns readable.  If the product does not
-    // complete within the wait bound the thread flags the error and stops waiting (its words are then wrong).
-    __device__ __forceinline__ void product(uint32_t off, uint32_t ksteps, uint32_t ld, uint32_t idesc)
+    // complete within the wait bound the thread flags the error and gives up: it waits for and issues nothing
+    // more, and its phase stays that of the product it gave up on, which finish() waits for once more.  It goes
+    // through the motions up to the end of the tile (the barriers need every thread; what a late product then
+    // reads from the rows no longer matters), stores no digest, and the group leaves at the next gave_up().
+    // `issue` and `limit` are for the probe of that path.
+    __device__ __forceinline__ void product(uint32_t off, uint32_t ksteps, uint32_t ld, uint32_t idesc, bool issue = true,
+                                            uint32_t limit = WAIT_LIMIT)
     {
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         sync();
-        if (issuer && !dead) {
+        if (issuer && !dead && issue) {
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             uint64_t a = matrix_desc(row, 2048), b = matrix_desc(tab + off, ld * 16);
             for (uint32_t k = 0; k < ksteps; k++) {
@@ -265,18 +288,23 @@ struct Group {
             }
             asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(mbar) : "memory");
         }
-        if (!dead && !wait(phase)) {
-            dead = true;
-            atomicExch(&g_tc_error, 1);
+        if (!dead) {
+            if (wait(limit)) {
+                phase ^= 1;
+            } else {
+                dead = true;
+                atomicExch(&g_tc_error, 1);
+            }
         }
-        phase ^= 1;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     }
 
     // Frees the tensor memory once every group is done with it.  All threads of the CTA.
-    __device__ __forceinline__ void finish(const Shared &sh)
+    __device__ __forceinline__ void finish(const Shared &sh, uint32_t limit = WAIT_LIMIT)
     {
-        if (dead) wait(phase ^ 1);  // give a late product one more bound to land
+        // A late product gets one more bound to land.  The issuer's wait covers every product issued: those before
+        // the one it gave up on it saw complete, and it has issued none since.
+        if (issuer && dead) wait(limit);
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         __syncthreads();
         if (threadIdx.x < 32) {
@@ -310,7 +338,7 @@ struct Group {
             }
         }
 #pragma unroll
-        for (int t = 0; t < N; t += 2) sts128(word_addr(W + first + t), y[t], t + 1 < N ? y[t + 1] : 0ull);
+        for (int t = 0; t < N; t += 2) store_row(W + first + t, y[t], t + 1 < N ? y[t + 1] : 0ull);
     }
 
     // The permutation of the states in the rows (Poseidon2: the state; Poseidon1: x^7 of the state plus the
@@ -343,7 +371,7 @@ struct Group {
                     for (int j = 0; j < 2; j++) x[j] = gl::mont_pow7(x[j]);
                 }
 #pragma unroll
-                for (int j = 0; j < 2; j += 2) sts128(word_addr(g + j), x[j], x[j + 1]);
+                for (int j = 0; j < 2; j += 2) store_row(g + j, x[j], x[j + 1]);
             }
         }
         product(S::OFF_F, S::KX / 32, S::NF, instr_desc(S::NF));
@@ -364,7 +392,7 @@ struct Group {
             a = gl::pow7(gl::add_c(a, k[g]));
             b = gl::pow7(gl::add_c(b, k[g + 1]));
         }
-        sts128(word_addr(g), a, b);
+        store_row(g, a, b);
     }
 };
 
@@ -400,7 +428,7 @@ __device__ __forceinline__ void leaf_tile(Group<W, FAM> &G, uint64_t *__restrict
         for (int i = 0; i < OUT; i += 2) G.put2(RATE + (int)G.half * OUT + i, cap[i], cap[i + 1]);
         G.permute(cap);
     }
-    if (valid) store_words(d, cap);
+    if (valid && !G.dead) store_words(d, cap);
 }
 
 // Parents of up to 128 nodes of one tree level (poseidon2_goldilocks.cpp:129-175): `pending` child digests at
@@ -432,7 +460,29 @@ __device__ __forceinline__ void node_tile(Group<W, FAM> &G, uint64_t *__restrict
     for (int j = 0; j < MINE; j += 2) G.put2((int)G.half * MINE + j, v[j], v[j + 1]);
     uint64_t o[OUT];
     G.permute(o);
-    if (i < parents) store_words(out + i * 4 + G.half * OUT, o);
+    if (i < parents && !G.dead) store_words(out + i * 4 + G.half * OUT, o);
+}
+
+// Probe of a product that does not complete: every group runs `before` products, waits a few rounds for one that is
+// never issued, and calls product `after` times more.  counts: threads that gave up; threads whose phase says the
+// missing product has landed; threads told to leave.
+__global__ void __launch_bounds__(Cfg<16>::THREADS, 1) product_wait_probe_kernel(uint32_t before, uint32_t after, uint32_t *counts)
+{
+    typedef Shape<16> S;
+    constexpr uint32_t LIMIT = 8;
+    extern __shared__ __align__(128) uint8_t tc_sm[];
+    __shared__ Shared sh;
+    Group<16, 2> G;
+    G.setup(tc_sm, sh);
+    if (G.half == 0)
+        for (int i = 0; i < 16; i += 2) G.store_row(i, 1, 2);
+    for (uint32_t i = 0; i < before; i++) G.product(S::OFF_L, S::KX / 32, S::KX, instr_desc(S::KX));
+    G.product(S::OFF_L, S::KX / 32, S::KX, instr_desc(S::KX), false, LIMIT);
+    for (uint32_t i = 0; i < after; i++) G.product(S::OFF_L, S::KX / 32, S::KX, instr_desc(S::KX));
+    atomicAdd(counts, G.dead ? 1u : 0u);
+    atomicAdd(counts + 1, G.wait(LIMIT) ? 1u : 0u);
+    atomicAdd(counts + 2, G.gave_up() ? 1u : 0u);
+    G.finish(sh, LIMIT);
 }
 
 // ------------------------------------------------------------------ host side ----
