@@ -331,8 +331,11 @@ uint64_t b200_launch_count(void);
  * Accelerator where the source is 16-byte aligned with an even column count, 0 always uses the
  * thread-loaded shared-memory tiles.  Same values either way; returns the previous setting. */
 int b200_set_transpose_tma(int on);
-/* 1 if a bounded wait ran out on the current device since the last call (a TMA transpose's tile copy or a
- * tensor core product of the hashing kernels; the flag is then reset), 0 otherwise, < 0 on a CUDA error. */
+/* Every wait inside a kernel is bounded (a TMA transpose's tile copy, a tensor core product of the hashing
+ * kernels).  One that runs out leaves wrong results, so from then on every call that waits for the device and
+ * hands on a root reports B200_ECUDA (get_stream_proofs: b200_buffers_error, and a zero root), until this call
+ * clears it: 1 if a wait ran out on the current device since the last call, 0 otherwise, < 0 on a CUDA error.
+ * After calls that do not wait (no root asked for), synchronise and look here. */
 int b200_tma_wait_errors(void);
 
 /* INT32 multiply-add throughput probe: `blocks` x 256 threads each run 8 independent

@@ -70,6 +70,12 @@ extern "C" int b200_batch_plan_run(void *plan_, uint64_t *roots_host, void *stre
     CK(plan->run(s, use_graph != 0), "batch run");
     if (roots_host) {
         CK(cudaStreamSynchronize(s), "batch sync");
+        int dev = 0, rc;
+        CK(cudaGetDevice(&dev), "cudaGetDevice");
+        if ((rc = wait_status(dev))) {
+            memset(roots_host, 0, 32 * plan->inst.size());
+            return rc;
+        }
         memcpy(roots_host, plan->h_roots, 32 * plan->inst.size());
     }
     return B200_OK;
@@ -91,7 +97,9 @@ extern "C" int b200_commit_batch_device(const B200BatchInstance *inst, uint64_t 
     int rc = b200_batch_plan_run(plan, roots_host, stream, 0);
     if (!rc && !roots_host) {
         cudaError_t e = cudaStreamSynchronize((cudaStream_t)stream);
-        if (e != cudaSuccess) rc = cuda_err(e, "batch sync");
+        int dev = 0;
+        if (e == cudaSuccess) e = cudaGetDevice(&dev);
+        rc = e != cudaSuccess ? cuda_err(e, "batch sync") : wait_status(dev);
     }
     b200_batch_plan_free(plan);
     return rc;

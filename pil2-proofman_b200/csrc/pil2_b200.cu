@@ -40,15 +40,16 @@ extern "C" const char *b200_last_error(void) { return t_err.c_str(); }
 
 // ------------------------------------------------------------- per device ----
 static std::mutex g_init_mu;
-static bool g_init_done[64];
+static bool g_init_done[wait_error::MAX_DEVICES];
 
 static int ensure_init_current()
 {
     int dev = 0;
     CK(cudaGetDevice(&dev), "cudaGetDevice");
-    if (dev < 0 || dev >= 64) return set_err(B200_EINVAL, "device index out of range");
+    if (dev < 0 || dev >= wait_error::MAX_DEVICES) return set_err(B200_EINVAL, "device index out of range");
     std::lock_guard<std::mutex> lk(g_init_mu);
     if (g_init_done[dev]) return B200_OK;
+    CK(wait_error::init(dev), "wait error word");
     CK(ntt::init_tables(), "ntt tables");
     CK(cudaFuncSetAttribute(ntt::pass16_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                             (NTT_TILE_MAX + NTT_TILE_MAX / 16) * 8),
@@ -60,6 +61,26 @@ static int ensure_init_current()
     CK(cudaStreamSynchronize(cudaStreamLegacy), "table upload");
     g_init_done[dev] = true;
     return B200_OK;
+}
+
+// After a synchronisation, before results are handed on: an error if a bounded wait of a kernel on device `dev` has
+// run out (the results may then be wrong).  Every call says so until b200_tma_wait_errors clears it.
+static int wait_status(int dev)
+{
+    if (!wait_error::raised(dev)) return B200_OK;
+    return set_err(B200_ECUDA, "a bounded wait of a kernel ran out on the device (b200_tma_wait_errors clears this)");
+}
+
+// the root of a tree whose last four words are at d_root, on `s`; waits for it
+static int root_to_host(uint64_t *root_host, const uint64_t *d_root, cudaStream_t s)
+{
+    int dev = 0;
+    CK(cudaGetDevice(&dev), "cudaGetDevice");
+    CK(cudaMemcpyAsync(root_host, d_root, 32, cudaMemcpyDeviceToHost, s), "root D2H");
+    CK(cudaStreamSynchronize(s), "sync");
+    const int rc = wait_status(dev);
+    if (rc) memset(root_host, 0, 32);
+    return rc;
 }
 
 extern "C" int b200_init(int device)
@@ -193,12 +214,7 @@ static int commit_device_fam(uint64_t *root_host, uint64_t *d_lde, uint64_t *d_t
     CK(ntt::lde(d_lde, d_trace, trace_rowmajor != 0, (uint32_t)nBits, (uint32_t)nBitsExt, nCols, d_scratch, s),
        "lde");
     CK(merkle::build_tree_arity(arity, d_tree, d_lde, 1, NExt, nCols, NExt, s, family), "merkletree");
-    if (root_host) {
-        const uint64_t total = merkle::tree_num_elements(NExt, arity);
-        CK(cudaMemcpyAsync(root_host, d_tree + total - 4, 32, cudaMemcpyDeviceToHost, s), "root D2H");
-        CK(cudaStreamSynchronize(s), "sync");
-    }
-    return B200_OK;
+    return root_host ? root_to_host(root_host, d_tree + merkle::tree_num_elements(NExt, arity) - 4, s) : B200_OK;
 }
 
 extern "C" int b200_commit_device(uint64_t *root_host, uint64_t *d_lde, uint64_t *d_tree, const uint64_t *d_trace,
@@ -596,10 +612,11 @@ static void harvest(CommitBuffers *b, Slot &s)
 {
     if (!s.busy) return;
     const cudaError_t e = cudaEventSynchronize(s.end);
-    if (e == cudaSuccess) {
+    const int rc = e == cudaSuccess ? wait_status(b->device) : cuda_err(e, "commit on the device");
+    if (!rc) {
         if (s.user_root) memcpy(s.user_root, s.h_root, 32);
     } else {
-        b->error = cuda_err(e, "commit on the device");
+        b->error = rc;
         if (s.user_root) memset(s.user_root, 0, 32);
     }
     s.busy = false;
@@ -949,6 +966,7 @@ extern "C" void write_custom_commit(void *root, uint64_t arity, uint64_t nBits, 
         rc = slot_commit(b, s, (const uint64_t *)buffer, nBits, nBitsExt, nCols, arity,
                          packed_layout(nBits, nBitsExt, nCols, arity));
         if (!rc && cudaStreamSynchronize(s.stream) != cudaSuccess) rc = set_err(B200_ECUDA, "commit failed");
+        if (!rc) rc = wait_status(b->device);
         if (!rc) memcpy(r, s.h_root, 32);
         if (!rc && bufferFile && bufferFile[0]) {
             std::vector<uint64_t> host((N + NExt) * nCols + tsz);
@@ -1020,7 +1038,10 @@ extern "C" void calculate_const_tree(void *pStarkInfo, void *pConstPolsAddress, 
     if (!rc && cudaMemcpyAsync(pConstTree, d_tree, total * 8, cudaMemcpyDeviceToHost, s) != cudaSuccess)
         rc = set_err(B200_ECUDA, "calculate_const_tree: result copy failed");
     // the stream is drained before the device buffers are freed, whatever happened above
-    if (cudaStreamSynchronize(s) != cudaSuccess && !rc) set_err(B200_ECUDA, "calculate_const_tree: commit failed");
+    int dev = 0;
+    if ((cudaStreamSynchronize(s) != cudaSuccess || cudaGetDevice(&dev) != cudaSuccess) && !rc)
+        rc = set_err(B200_ECUDA, "calculate_const_tree: commit failed");
+    if (!rc) wait_status(dev);
     cudaStreamDestroy(s);
 }
 
@@ -1044,16 +1065,14 @@ extern "C" uint64_t b200_launch_count(void) { return prof::g_launches.load(); }
 
 extern "C" int b200_set_transpose_tma(int on) { return ntt::transpose_tma_enabled().exchange(on ? 1 : 0); }
 
-// the bounded waits' error flags on the current device (1: a TMA tile copy or a tensor core product did not
-// complete within the kernel's wait bound), reset to 0
+// the bounded waits' error word on the current device (1: a TMA tile copy or a tensor core product did not
+// complete within the kernel's wait bound), cleared
 extern "C" int b200_tma_wait_errors(void)
 {
-    int v = 0, w = 0, zero = 0;
-    if (cudaMemcpyFromSymbol(&v, g_tma_error, sizeof(int)) != cudaSuccess) return cuda_err(cudaGetLastError(), "flag");
-    if (cudaMemcpyFromSymbol(&w, g_tc_error, sizeof(int)) != cudaSuccess) return cuda_err(cudaGetLastError(), "flag");
-    CK(cudaMemcpyToSymbol(g_tma_error, &zero, sizeof(int)), "flag reset");
-    CK(cudaMemcpyToSymbol(g_tc_error, &zero, sizeof(int)), "flag reset");
-    return v | w;
+    int dev = 0;
+    CK(cudaGetDevice(&dev), "cudaGetDevice");
+    CK(cudaStreamSynchronize(cudaStreamLegacy), "flag");
+    return wait_error::clear(dev) ? 1 : 0;
 }
 
 __global__ void __launch_bounds__(256) imad_probe_kernel(uint32_t *out, uint64_t iters, uint32_t seed)
@@ -1161,12 +1180,7 @@ extern "C" int b200_commit_q_device(uint64_t *root_host, uint64_t *d_cmq, uint64
                   d_scratch, s),
        "Q extension");
     CK(merkle::build_tree_arity(arity, d_tree, d_cmq, 1, NExt, ncols, NExt, s, g_native_family.load()), "merkletree");
-    if (root_host) {
-        const uint64_t total = merkle::tree_num_elements(NExt, arity);
-        CK(cudaMemcpyAsync(root_host, d_tree + total - 4, 32, cudaMemcpyDeviceToHost, s), "root D2H");
-        CK(cudaStreamSynchronize(s), "sync");
-    }
-    return B200_OK;
+    return root_host ? root_to_host(root_host, d_tree + merkle::tree_num_elements(NExt, arity) - 4, s) : B200_OK;
 }
 
 // ------------------------------------------------------------ plan autotuner ----
@@ -1343,12 +1357,7 @@ extern "C" int b200_commit_packed_device(uint64_t *root_host, uint64_t *d_lde, u
         CK(ntt::lde(d_lde, d_scratch, false, (uint32_t)nBits, (uint32_t)nBitsExt, nCols, d_scratch, s), "lde");
     }
     CK(merkle::build_tree_arity(arity, d_tree, d_lde, 1, NExt, nCols, NExt, s, g_native_family.load()), "merkletree");
-    if (root_host) {
-        const uint64_t total = merkle::tree_num_elements(NExt, arity);
-        CK(cudaMemcpyAsync(root_host, d_tree + total - 4, 32, cudaMemcpyDeviceToHost, s), "root D2H");
-        CK(cudaStreamSynchronize(s), "sync");
-    }
-    return B200_OK;
+    return root_host ? root_to_host(root_host, d_tree + merkle::tree_num_elements(NExt, arity) - 4, s) : B200_OK;
 }
 
 // ------------------------------------------------------ streaming slot commit ----
@@ -1424,9 +1433,7 @@ static int stream_commit_on(uint64_t *slot, uint64_t slot_words, cudaStream_t s,
                    : stream::run<2>(slot, l, nBits, nBitsExt, nCols, wordsPerRow, s, px),
        "streaming commit");
     const uint64_t tsz = merkle::tree_num_elements(NExt, 4);
-    CK(cudaMemcpyAsync(root, slot + l.tree + tsz - 4, 32, cudaMemcpyDeviceToHost, s), "root D2H");
-    CK(cudaStreamSynchronize(s), "sync");
-    return B200_OK;
+    return root_to_host(root, slot + l.tree + tsz - 4, s);
 }
 
 extern "C" uint64_t stream_commit_slot_bytes(uint64_t nBits, uint64_t nBitsExt, uint64_t nCols, uint64_t wordsPerRow)
@@ -1638,12 +1645,7 @@ extern "C" int b200_commit_indexed_device(uint64_t *root_host, uint64_t *d_lde, 
         CK(ntt::lde(d_lde, d_scratch, false, (uint32_t)nBits, (uint32_t)nBitsExt, nCols, d_scratch, s), "lde");
     }
     CK(merkle::build_tree_arity(arity, d_tree, d_lde, 1, NExt, nCols, NExt, s, g_native_family.load()), "merkletree");
-    if (root_host) {
-        const uint64_t total = merkle::tree_num_elements(NExt, arity);
-        CK(cudaMemcpyAsync(root_host, d_tree + total - 4, 32, cudaMemcpyDeviceToHost, s), "root D2H");
-        CK(cudaStreamSynchronize(s), "sync");
-    }
-    return B200_OK;
+    return root_host ? root_to_host(root_host, d_tree + merkle::tree_num_elements(NExt, arity) - 4, s) : B200_OK;
 }
 
 // Native streaming commit of an indexed witness (host rows, device table).

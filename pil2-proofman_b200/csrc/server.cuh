@@ -462,6 +462,8 @@ class Server {
     // results of a finished unit to its requests; frees the unit (caller holds mu)
     void finish_unit(Unit *u, bool ok)
     {
+        const bool waits_held = !wait_error::raised(device);
+        ok = ok && waits_held;
         const double t = now_ms();
         const double gi = ok ? since_t0(u->issued) : -1, gc = ok ? since_t0(u->copied) : -1,
                      gs = ok ? since_t0(u->started) : -1, gd = ok ? since_t0(u->done) : -1;
@@ -481,7 +483,8 @@ class Server {
                 used -= 8 * 2 * r->words_trace;
             } else {
                 r->status = B200_ECUDA;
-                r->err = "request failed on the device (CUDA error)";
+                r->err = waits_held ? "request failed on the device (CUDA error)"
+                                    : "a bounded wait of a kernel ran out on the device";
                 free_buffers(r);
                 used -= r->bytes();
             }

@@ -22,8 +22,7 @@
 #pragma once
 #include "gl64.cuh"
 #include "tc_tables.h"
-
-__device__ int g_tc_error;  // set when a product did not complete within the wait bound
+#include "wait_error.cuh"
 
 // Table bytes and constants by [family - 1][width / 4 - 2], uploaded once per device.
 __device__ __align__(16) uint8_t g_tc_tab[2][3][tch::MAX_BYTES];
@@ -293,7 +292,7 @@ struct Group {
                 phase ^= 1;
             } else {
                 dead = true;
-                atomicExch(&g_tc_error, 1);
+                wait_error::raise();
             }
         }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");

@@ -23,8 +23,7 @@
 #include <mutex>
 
 #include "prof.cuh"
-
-__device__ int g_tma_error;  // set when a tile copy did not land within the wait bound
+#include "wait_error.cuh"
 
 namespace ntt {
 
@@ -74,7 +73,7 @@ __global__ void __launch_bounds__(256) transpose_tma_kernel(uint64_t *__restrict
     }
     __syncthreads();  // the barrier is initialised before anyone waits on it
     if (!mbar_wait_bounded(mbar, 0)) {
-        if (tx == 0 && ty == 0) atomicExch(&g_tma_error, 1);
+        if (tx == 0 && ty == 0) wait_error::raise();
         return;
     }
     const uint64_t r = r0 + tx;
