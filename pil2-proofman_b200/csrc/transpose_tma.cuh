@@ -10,7 +10,7 @@
 // chunk positions instead of one bank.  Every thread then writes 4 columns x 32 consecutive rows:
 // 256-byte coalesced stores.  Out-of-range rows and columns of edge tiles are zero-filled by the
 // copy and skipped by the stores.  The wait on the barrier is bounded: if the copy never lands the
-// CTA records an error flag and returns instead of spinning.
+// CTA raises the error word, gives it one more bound and returns instead of spinning.
 //
 // Preconditions (checked by the host dispatcher, which otherwise uses ntt::transpose_kernel): the
 // source 16-byte aligned, its row pitch nCols * 8 a multiple of 16 bytes (nCols even), and the
@@ -74,6 +74,7 @@ __global__ void __launch_bounds__(256) transpose_tma_kernel(uint64_t *__restrict
     __syncthreads();  // the barrier is initialised before anyone waits on it
     if (!mbar_wait_bounded(mbar, 0)) {
         if (tx == 0 && ty == 0) wait_error::raise();
+        mbar_wait_bounded(mbar, 0);  // the late copy writes this CTA's memory: one more bound to land in
         return;
     }
     const uint64_t r = r0 + tx;
