@@ -193,13 +193,15 @@ __global__ void __launch_bounds__(tch::Cfg<W>::THREADS, 1)
 }
 
 template <int W, int FAM>
-__global__ void __launch_bounds__(tch::Cfg<W>::THREADS, 1) node_grouped(const NodeEntry *e, int n, uint64_t total)
+__global__ void __launch_bounds__(tch::Cfg<W>::THREADS, 1) node_grouped(const NodeEntry *e, int n, uint64_t total,
+                                                                        tch::Split split)
 {
     extern __shared__ __align__(128) uint8_t tc_sm[];
     __shared__ tch::Shared sh;
     tch::Group<W, FAM> G;
     G.setup(tc_sm, sh);
-    for (uint64_t b = blockIdx.x + (uint64_t)gridDim.x * G.id; b < total; b += (uint64_t)gridDim.x * tch::Cfg<W>::GROUPS) {
+    const tch::TileRange<W> r(split, G.id, total);
+    for (uint64_t b = r.first; b < r.end; b += r.step) {
         const NodeEntry &E = e[find_entry(e, n, b)];
         tch::node_tile(G, E.level, E.pending, E.pad, E.parents, E.out, b - E.begin);
         if (G.gave_up()) break;
@@ -609,16 +611,19 @@ class Plan {
                 break;
             }
             case 3: {
-                const unsigned ctas = (unsigned)std::min<uint64_t>(L.blocks, (uint64_t)leaf_ctas);
+                const uint64_t sms = (uint64_t)leaf_ctas;
+                const tch::Split split = L.width == 8    ? tch::split<8>(L.blocks, 1, sms)
+                                         : L.width == 12 ? tch::split<12>(L.blocks, 1, sms)
+                                                         : tch::split<16>(L.blocks, 1, sms);
                 const NodeEntry *ne = (const NodeEntry *)ent;
                 if (family == 1) {
-                    if (L.width == 8) node_grouped<8, 1><<<ctas, tch::Cfg<8>::THREADS, tch::Smem<8>::BYTES, s>>>(ne, L.n, L.blocks);
-                    if (L.width == 12) node_grouped<12, 1><<<ctas, tch::Cfg<12>::THREADS, tch::Smem<12>::BYTES, s>>>(ne, L.n, L.blocks);
-                    if (L.width == 16) node_grouped<16, 1><<<ctas, tch::Cfg<16>::THREADS, tch::Smem<16>::BYTES, s>>>(ne, L.n, L.blocks);
+                    if (L.width == 8) node_grouped<8, 1><<<split.ctas, tch::Cfg<8>::THREADS, tch::Smem<8>::BYTES, s>>>(ne, L.n, L.blocks, split);
+                    if (L.width == 12) node_grouped<12, 1><<<split.ctas, tch::Cfg<12>::THREADS, tch::Smem<12>::BYTES, s>>>(ne, L.n, L.blocks, split);
+                    if (L.width == 16) node_grouped<16, 1><<<split.ctas, tch::Cfg<16>::THREADS, tch::Smem<16>::BYTES, s>>>(ne, L.n, L.blocks, split);
                 } else {
-                    if (L.width == 8) node_grouped<8, 2><<<ctas, tch::Cfg<8>::THREADS, tch::Smem<8>::BYTES, s>>>(ne, L.n, L.blocks);
-                    if (L.width == 12) node_grouped<12, 2><<<ctas, tch::Cfg<12>::THREADS, tch::Smem<12>::BYTES, s>>>(ne, L.n, L.blocks);
-                    if (L.width == 16) node_grouped<16, 2><<<ctas, tch::Cfg<16>::THREADS, tch::Smem<16>::BYTES, s>>>(ne, L.n, L.blocks);
+                    if (L.width == 8) node_grouped<8, 2><<<split.ctas, tch::Cfg<8>::THREADS, tch::Smem<8>::BYTES, s>>>(ne, L.n, L.blocks, split);
+                    if (L.width == 12) node_grouped<12, 2><<<split.ctas, tch::Cfg<12>::THREADS, tch::Smem<12>::BYTES, s>>>(ne, L.n, L.blocks, split);
+                    if (L.width == 16) node_grouped<16, 2><<<split.ctas, tch::Cfg<16>::THREADS, tch::Smem<16>::BYTES, s>>>(ne, L.n, L.blocks, split);
                 }
                 break;
             }

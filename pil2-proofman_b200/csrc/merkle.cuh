@@ -46,22 +46,21 @@ __device__ __forceinline__ void permute_fam(uint64_t *st)
         p2::permute_smem<W, TPB>(st);
 }
 
-// Row sponges of `nrows` rows, 128-row tiles over the groups of every CTA (tc_hash.cuh), tile t to CTA t mod the
-// grid first so that few tiles spread over the SMs.  Against one thread a row with the state in shared memory and
+// Row sponges of `nrows` rows, 128-row tiles over the groups of every CTA (tc_hash.cuh).  Against one thread a row with the state in shared memory and
 // every layer on the integer pipes, 2^20 rows (B200): Poseidon2 W16 x 256 columns 24.6 -> 16.4 ms (937 -> 1403 M
 // permutations/s), W12 x 128 13.9 -> 9.8, W8 x 64 9.6 -> 7.0; Poseidon1 W16 39.0 -> 16.4, W12 19.4 -> 9.7, W8 12.5 -> 7.0.
 template <int W, int FAM = 2>
 __global__ void __launch_bounds__(tch::Cfg<W>::THREADS, 1) leaf_hash_kernel(uint64_t *__restrict__ digests,
                                                                     const uint64_t *__restrict__ src, uint64_t rs,
                                                                     uint64_t cs, uint64_t ncols, uint64_t nrows,
-                                                                    int resume)
+                                                                    int resume, tch::Split split)
 {
     extern __shared__ __align__(128) uint8_t tc_sm[];
     __shared__ tch::Shared sh;
     tch::Group<W, FAM> G;
     G.setup(tc_sm, sh);
-    const uint64_t tiles = (nrows + 127) / 128;
-    for (uint64_t t = blockIdx.x + (uint64_t)gridDim.x * G.id; t < tiles; t += (uint64_t)gridDim.x * tch::Cfg<W>::GROUPS) {
+    const tch::TileRange<W> r(split, G.id, (nrows + 127) / 128);
+    for (uint64_t t = r.first; t < r.end; t += r.step) {
         tch::leaf_tile(G, digests, src, rs, cs, ncols, nrows, t, resume != 0);
         if (G.gave_up()) break;
     }
@@ -71,14 +70,15 @@ __global__ void __launch_bounds__(tch::Cfg<W>::THREADS, 1) leaf_hash_kernel(uint
 // One tree level of `parents` parents.
 template <int W, int FAM = 2>
 __global__ void __launch_bounds__(tch::Cfg<W>::THREADS, 1) node_kernel(uint64_t *__restrict__ level, uint64_t pending, uint64_t pad,
-                                                               uint64_t parents, uint64_t *__restrict__ out)
+                                                               uint64_t parents, uint64_t *__restrict__ out,
+                                                               tch::Split split)
 {
     extern __shared__ __align__(128) uint8_t tc_sm[];
     __shared__ tch::Shared sh;
     tch::Group<W, FAM> G;
     G.setup(tc_sm, sh);
-    const uint64_t tiles = (parents + 127) / 128;
-    for (uint64_t t = blockIdx.x + (uint64_t)gridDim.x * G.id; t < tiles; t += (uint64_t)gridDim.x * tch::Cfg<W>::GROUPS) {
+    const tch::TileRange<W> r(split, G.id, (parents + 127) / 128);
+    for (uint64_t t = r.first; t < r.end; t += r.step) {
         tch::node_tile(G, level, pending, pad, parents, out, t);
         if (G.gave_up()) break;
     }
@@ -145,8 +145,9 @@ cudaError_t build_levels(uint64_t *d_tree, uint64_t nrows, cudaStream_t stream)
             prof::count();
             continue;
         }
-        node_kernel<W, FAM><<<tch::grid((parents + 127) / 128), tch::Cfg<W>::THREADS, tch::Smem<W>::BYTES, stream>>>(
-            lvl, pending, pad, parents, lvl + (pending + pad) * 4);
+        const tch::Split split = tch::split<W>((parents + 127) / 128, 1);
+        node_kernel<W, FAM><<<split.ctas, tch::Cfg<W>::THREADS, tch::Smem<W>::BYTES, stream>>>(
+            lvl, pending, pad, parents, lvl + (pending + pad) * 4, split);
         prof::count();
         base += (pending + pad) * 4;
         pending = parents;
@@ -159,8 +160,9 @@ template <int W, int FAM = 2>
 cudaError_t hash_rows(uint64_t *digests, const uint64_t *src, uint64_t rs, uint64_t cs, uint64_t ncols, uint64_t nrows,
                       bool resume, cudaStream_t stream)
 {
-    leaf_hash_kernel<W, FAM><<<tch::grid((nrows + 127) / 128), tch::Cfg<W>::THREADS, tch::Smem<W>::BYTES, stream>>>(
-        digests, src, rs, cs, ncols, nrows, resume ? 1 : 0);
+    const tch::Split split = tch::split<W>((nrows + 127) / 128, (ncols + W - 5) / (W - 4));
+    leaf_hash_kernel<W, FAM><<<split.ctas, tch::Cfg<W>::THREADS, tch::Smem<W>::BYTES, stream>>>(
+        digests, src, rs, cs, ncols, nrows, resume ? 1 : 0, split);
     prof::count();
     return cudaGetLastError();
 }

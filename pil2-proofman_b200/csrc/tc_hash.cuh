@@ -395,6 +395,25 @@ struct Group {
     }
 };
 
+// Tiles of a launch over its CTAs: waves of `lanes` CTAs, `rounds` tiles a group and wave; a wave's first tiles go
+// to different CTAs, so that few tiles spread over the SMs.
+struct Split {
+    uint32_t lanes, rounds, ctas;
+};
+
+// A group's tiles: for (t = first; t < end; t += step).
+template <int W>
+struct TileRange {
+    uint64_t first, end, step;
+    __device__ __forceinline__ TileRange(const Split &s, uint32_t group, uint64_t tiles)
+    {
+        step = (uint64_t)s.lanes * Cfg<W>::GROUPS;
+        const uint64_t wave = step * s.rounds, begin = blockIdx.x / s.lanes * wave;
+        first = begin + (uint64_t)group * s.lanes + blockIdx.x % s.lanes;
+        end = tiles - begin < wave ? tiles : begin + wave;
+    }
+};
+
 // Row sponge of up to 128 rows (capacity zeroed at the start; every block of RATE columns overwrites words
 // [0, RATE), zero past the last column, and carries words [0, 4) into the capacity; 0 columns give the zero digest:
 // poseidon2_goldilocks.cpp:42-77).  `resume`: the digests hold the four words of the blocks before.  Threads past the last
@@ -514,14 +533,31 @@ inline cudaError_t init_tables()
     return upload<16>();
 }
 
-// CTAs of a launch over `tiles` 128-row tiles: one an SM, no more than tiles
-inline unsigned grid(uint64_t tiles)
+// Launch over `tiles` 128-row tiles of `perms` permutations a row.  A CTA holds its SM to its end, and a kernel of a
+// higher-priority stream enters at CTA ends only, so a group takes the tiles of 16 permutations (0.9-1.0 ms with every
+// group at work) or one wider tile, and the next CTA goes on.  With one CTA an SM for all tiles, query openings issued
+// at high priority 1 ms into a tree of 2^20 x 256 waited 14.9 ms (whole sponge 16.4), with these 0.08; the trees take the
+// same (16.60 and 16.61 ms; 2^20 x 24: 1.86 both).  Half as many permutations a CTA take 2 % more at 24 columns: a table
+// load and tensor memory setup are a few microseconds each.
+constexpr uint64_t CTA_PERMS = 16;
+template <int W>
+inline Split split(uint64_t tiles, uint64_t perms, uint64_t sms)
+{
+    const uint64_t rounds = perms >= CTA_PERMS ? 1 : perms ? CTA_PERMS / perms : CTA_PERMS;
+    const uint64_t lanes = tiles < sms ? tiles : sms, wave = rounds * Cfg<W>::GROUPS * lanes;
+    const uint64_t rest = tiles % wave;
+    return Split{(uint32_t)lanes, (uint32_t)rounds, (uint32_t)(tiles / wave * lanes + (rest < lanes ? rest : lanes))};
+}
+
+// the same on the current device
+template <int W>
+inline Split split(uint64_t tiles, uint64_t perms)
 {
     int dev = 0, sms = 0;
     if (cudaGetDevice(&dev) != cudaSuccess ||
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms < 1)
         sms = 1;
-    return (unsigned)(tiles < (uint64_t)sms ? tiles : (uint64_t)sms);
+    return split<W>(tiles, perms, (uint64_t)sms);
 }
 
 }  // namespace tch

@@ -57,6 +57,24 @@ def test_tree_at_the_tiles_edges(dev, arity, family, nrows):
         assert bad.size == 0, (nrows, ncols, arity, family, bad[:8])
 
 
+# One tile past a whole wave of CTAs that take a single tile a group (16 permutations a row and more), and past one of
+# CTAs that take two (8 permutations): the next wave's first CTA, with one group at work.
+@pytest.mark.parametrize("arity,nrows,blocks", [(4, 148 * 4 * 128 + 1, 17), (2, 148 * 8 * 128 + 1, 16),
+                                                (3, 2 * 148 * 4 * 128 + 1, 8)])
+def test_tree_past_a_wave(dev, orc, arity, nrows, blocks):
+    pkg, torch = dev
+    pkg.set_native_hash_family(2)
+    ncols = blocks * (4 * arity - 4) - 1
+    m = oracle.random_field((nrows, ncols), nrows)
+    exp = orc.merkletree(m, arity)
+    d_src = torch.from_numpy(np.ascontiguousarray(m.T).view(np.int64)).cuda()
+    tree = torch.zeros(exp.size, dtype=torch.int64, device="cuda")
+    pkg.merkletree_device(tree, d_src, 1, nrows, ncols, nrows, arity)
+    torch.cuda.synchronize()
+    bad = np.nonzero(tree.cpu().numpy().view(np.uint64) != exp)[0]
+    assert bad.size == 0, bad[:8]
+
+
 # Levels by subtrees of the tree (coop.cuh): one CTA's last parent and one more (16, 9, 32 parents at arity 4, 3, 2), a
 # launch's top level ending on one digest or leaving two, and missing children at every level.
 LEVELS = [(4, n) for n in (2, 4, 5, 63, 64, 65, 255, 257, 1025, 4096, 4099, 16384)] + \
