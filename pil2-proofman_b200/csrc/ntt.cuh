@@ -814,12 +814,22 @@ inline void set_tuned(uint32_t nBits, uint32_t nBitsExt, uint64_t ncols, Tune t)
     tune_table()[tune_key(nBits, nBitsExt, ncols)] = t;
 }
 
-// Windows covering stages [lo, hi).  The window that starts at `lo` keeps every lower lane (lgL = lo) if that fills a
-// tile, so its tile is one contiguous run, and else takes one lane (2^9 rows x 19 columns at blowup 2: 24.8 us
-// in the runtime-shaped kernel, the whole LDE 37 -> 27 us with the fixed one); the others take as many lanes as fill an
+// Whether a first window of 2^k points, of transforms of 2^hi, that fills no tile with its copy lanes takes one lane a
+// CTA, in the fixed-shape kernels, rather than all of them in one contiguous tile of the runtime-shaped one.  Per element
+// the fixed kernel is faster, but it takes more CTAs, whose words are lanes apart.  Measured for whole transforms of
+// k = 1..11 stages at every blowup and 2^8 to 2^17 CTAs, all lanes against one: from 2^9 points 1.12-1.35x at any
+// number; from 2^5, 1.00-2.3x up to 4096 CTAs and 0.4-1.0x from 16384 (2^5 -> 2^12 x 512 columns: 35 us against 66);
+// below, 1.0-2.0x up to 2048 and 0.2-1.2x past 4096 (2^1 -> 2^8 x 512: 10.5 us against 41).
+inline bool one_lane(uint32_t k, uint32_t hi, uint64_t ncols)
+{
+    return k >= 9 || ncols << (hi - k) <= (k >= 5 ? 4096u : 2048u);
+}
+
+// Windows covering stages [lo, hi) of `ncols` columns.  The window that starts at `lo` keeps every lower lane (lgL = lo),
+// so its tile is one contiguous run, or takes one lane (one_lane); the others take as many lanes as fill an
 // 8192-element tile (at most all 2^s0 of them).  kfirst / krest cap the first window and the
 // others (the autotuned plan parameters).
-inline int plan_windows(uint32_t lo, uint32_t hi, Window *w, int maxw, uint32_t kfirst = NTT_KMAX,
+inline int plan_windows(uint32_t lo, uint32_t hi, uint64_t ncols, Window *w, int maxw, uint32_t kfirst = NTT_KMAX,
                         uint32_t krest = 11)
 {
     int n = 0;
@@ -830,8 +840,7 @@ inline int plan_windows(uint32_t lo, uint32_t hi, Window *w, int maxw, uint32_t 
     if (k0 + lo > 13) k0 = (lo >= 13) ? 0 : 13 - lo;
     if (k0 == 0 && total > 0) return -1;  // stage offset too large for one tile
     if (krest < 1 || krest > NTT_KMAX) krest = 11;
-    // a first window that fills no tile takes one lane of the 2^lo copies a CTA: that shape has a fixed kernel
-    w[n++] = Window{lo, k0, k0 + lo == 13 ? lo : 0};
+    w[n++] = Window{lo, k0, k0 + lo == 13 || !one_lane(k0, hi, ncols) ? lo : 0};
     uint32_t rest = total - k0, s = lo + k0;
     uint32_t np = (rest + krest - 1) / krest;
     for (uint32_t i = 0; i < np; i++) {
@@ -893,7 +902,7 @@ inline cudaError_t lde(uint64_t *d_lde, const uint64_t *d_trace, bool trace_rowm
     // inverse DIF over [0, nBits), windows applied from the top stage down
     Window w[8];
     const Tune tn = tuned(nBits, nBitsExt, ncols);
-    int nw = nBits ? plan_windows(0, nBits, w, 8, tn.kfirst, tn.krest) : 0;
+    int nw = nBits ? plan_windows(0, nBits, ncols, w, 8, tn.kfirst, tn.krest) : 0;
     if (nw < 0) return cudaErrorInvalidValue;
     {
     prof::Scope ps(prof::NTT_INV, stream);
@@ -917,7 +926,7 @@ inline cudaError_t lde(uint64_t *d_lde, const uint64_t *d_trace, bool trace_rowm
     }
 
     // forward DIT over [b, nBitsExt) with replication by 2^b on the first window
-    nw = plan_windows(b, nBitsExt, w, 8, tn.kfirst, tn.krest);
+    nw = plan_windows(b, nBitsExt, ncols, w, 8, tn.kfirst, tn.krest);
     if (nw < 0) return cudaErrorInvalidValue;
     prof::Scope ps(prof::NTT_FWD, stream);
     for (int i = 0; i < nw; i++) {
@@ -966,7 +975,7 @@ inline cudaError_t lde_q(uint64_t *d_cmq, const uint64_t *d_q, bool q_rowmajor, 
     if ((err = cudaGetLastError()) != cudaSuccess) return err;
     Window w[8];
     const Tune tn = tuned(nBitsExt, nBitsExt, qDim);
-    int nw = plan_windows(0, nBitsExt, w, 8, tn.kfirst, tn.krest);
+    int nw = plan_windows(0, nBitsExt, qDim, w, 8, tn.kfirst, tn.krest);
     if (nw < 0) return cudaErrorInvalidValue;
     {
         prof::Scope ps(prof::NTT_INV, stream);
@@ -984,7 +993,7 @@ inline cudaError_t lde_q(uint64_t *d_cmq, const uint64_t *d_q, bool q_rowmajor, 
             if ((err = launch_pass(p, qDim, stream)) != cudaSuccess) return err;
         }
     }
-    nw = plan_windows(b, nBitsExt, w, 8, tn.kfirst, tn.krest);
+    nw = plan_windows(b, nBitsExt, qDim, w, 8, tn.kfirst, tn.krest);
     if (nw < 0) return cudaErrorInvalidValue;
     prof::Scope ps(prof::NTT_FWD, stream);
     const uint64_t shift_in = glh::pow(glh::inv(7), N), next_inv = glh::inv(NExt % GL_P);

@@ -1239,10 +1239,10 @@ extern "C" int b200_autotune_lde(uint64_t nBits, uint64_t nBitsExt, uint64_t nCo
     auto windows = [&](ntt::Tune t) {
         std::vector<uint32_t> v;
         ntt::Window w[8];
-        int n1 = nBits ? ntt::plan_windows(0, (uint32_t)nBits, w, 8, t.kfirst, t.krest) : 0;
+        int n1 = nBits ? ntt::plan_windows(0, (uint32_t)nBits, probe, w, 8, t.kfirst, t.krest) : 0;
         for (int i = 0; i < n1; i++) v.insert(v.end(), {w[i].s0, w[i].k, w[i].lgL});
         v.push_back(99);
-        int n2 = ntt::plan_windows((uint32_t)(nBitsExt - nBits), (uint32_t)nBitsExt, w, 8, t.kfirst, t.krest);
+        int n2 = ntt::plan_windows((uint32_t)(nBitsExt - nBits), (uint32_t)nBitsExt, probe, w, 8, t.kfirst, t.krest);
         for (int i = 0; i < n2; i++) v.insert(v.end(), {w[i].s0, w[i].k, w[i].lgL});
         if (n1 < 0 || n2 < 0) v.clear();
         return v;

@@ -46,3 +46,51 @@ def test_lde_over_all_words(dev, orc, nbits, nbits_ext):
     torch.cuda.synchronize()
     got = d_lde.cpu().numpy().view(np.uint64).T
     assert (got == exp).all(), (nbits, nbits_ext, np.argwhere(got != exp)[:4])
+
+
+# Both sides of the rule for first windows that fill no tile (one copy lane a CTA, or all of them): 2048 CTAs below 2^5
+# points, 4096 from there, no limit from 2^9.
+EDGES = [(1, 8, 16), (1, 8, 17), (2, 4, 512), (2, 4, 513), (4, 8, 128), (4, 8, 129), (5, 12, 32), (5, 12, 33), (8, 12, 256),
+         (8, 12, 257), (9, 12, 513)]
+
+
+@pytest.mark.parametrize("nbits,nbits_ext,ncols", EDGES)
+def test_lde_at_the_lane_rule(dev, orc, nbits, nbits_ext, ncols):
+    pkg, torch = dev
+    rng = np.random.RandomState(nbits * 31 + ncols)
+    m = rng.randint(0, 1 << 63, (1 << nbits, ncols)).astype(np.uint64) * np.uint64(2) + np.uint64(1)
+    m[:, ::3] = np.uint64(2**64 - 1)
+    m[::2, 1::3] = np.uint64(oracle.P)
+    exp = orc.lde(m % np.uint64(oracle.P), nbits_ext)
+    d_trace = torch.from_numpy(np.ascontiguousarray(m).view(np.int64)).cuda()
+    d_lde = torch.full((ncols, 1 << nbits_ext), -1, dtype=torch.int64, device="cuda")
+    d_scr = torch.empty(pkg.lde_scratch_words(nbits, ncols), dtype=torch.int64, device="cuda")
+    pkg.lde_device(d_lde, d_trace, nbits, nbits_ext, ncols, d_scr)
+    torch.cuda.synchronize()
+    got = d_lde.cpu().numpy().view(np.uint64).T
+    assert (got == exp).all(), np.argwhere(got != exp)[:4]
+
+
+def test_few_rows_at_a_high_blowup_take_no_longer(dev):
+    """2^1 -> 2^8 writes what 2^7 -> 2^8 does with fewer stages; with a CTA of two points a copy lane it took three times
+    as long (41 us against 13).  Best of several runs each."""
+    pkg, torch = dev
+    ncols, next_ = 512, 1 << 8
+    lde = torch.empty(ncols * next_, dtype=torch.int64, device="cuda")
+
+    def best(nbits):
+        trace = torch.zeros(ncols << nbits, dtype=torch.int64, device="cuda")
+        scr = torch.empty(pkg.lde_scratch_words(nbits, ncols), dtype=torch.int64, device="cuda")
+        ms = []
+        for _ in range(8):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            for _ in range(20):
+                pkg.lde_device(lde, trace, nbits, 8, ncols, scr, trace_rowmajor=False)
+            b.record()
+            torch.cuda.synchronize()
+            ms.append(a.elapsed_time(b))
+        return min(ms[1:])
+
+    few, many = best(1), best(7)
+    assert few < 1.5 * many, (few, many)
