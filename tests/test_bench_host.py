@@ -1,9 +1,12 @@
 """Host-side pieces of bench.py that need no GPU: the served stream's device-timeline split, the
 C3 / c3small shape draws, and the reference arm's step bound.  (The timed legs themselves are GPU
 work and are checked by running bench.py on a B200.)"""
+import argparse
+import json
 import os
 import sys
 
+import numpy as np
 import pytest
 
 REPO = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
@@ -47,3 +50,29 @@ def test_c3_shape_draws():
 def test_reference_arm_step_bound():
     assert bench.REF_MAX_STEPS >= 1
     assert max(1, min(20, bench.REF_MAX_STEPS)) == bench.REF_MAX_STEPS
+
+
+def _without_reference_build(monkeypatch):
+    def absent(*a, **k):
+        raise FileNotFoundError("oracle/_ref")
+    monkeypatch.setattr(bench, "time_reference_cpu", absent)
+    for k in ("RANK", "WORLD_SIZE", "LOCAL_RANK"):
+        monkeypatch.delenv(k, raising=False)
+    return argparse.Namespace(gpus=1, steps=2, warmup=3, hash_family=2, workload="c1", no_cpu_baseline=False,
+                              no_legs=True)
+
+
+def test_reference_arm_without_the_reference_build(monkeypatch, capsys):
+    args = _without_reference_build(monkeypatch)
+    assert bench.run_reference(args, bench.WORKLOADS["c1"]) == 0
+    line = json.loads(capsys.readouterr().out)
+    assert line["impl"] == "reference" and "oracle/_ref" in line["unavailable"]
+
+
+def test_own_arm_without_the_reference_build(monkeypatch, capsys):
+    args = _without_reference_build(monkeypatch)
+    monkeypatch.setattr(bench, "full_size_fixture", lambda *a: None)
+    roots = [np.arange(4, dtype=np.uint64)]
+    assert bench.finish(args, bench.WORKLOADS["c1"], None, None, 0, 1, 12.5, 20.0, 7, {}, {}, {}, roots, None) == 0
+    line = json.loads(capsys.readouterr().out)
+    assert line["value"] == 12.5 and line["gpu_launches"] == 7 and "oracle/_ref" in line["cpu_baseline"]["unavailable"]
