@@ -197,28 +197,19 @@ __device__ __forceinline__ uint64_t sub_c(uint64_t a, uint64_t b)
     return mk64(s0, s1);
 }
 
-// x * 2^S mod p for 0 < S < 96 by shifts: x << S spans at most three 32-bit words placed at word
+// x * 2^S mod p for 0 < S < 32 and 64 < S < 96 by shifts: x << S spans at most three 32-bit words placed at word
 // offset S/32, folded with 2^64 = 2^32 - 1, 2^96 = -1 and 2^128 = -2^32 (mod p).  At offset 0 the
 // words are (u1:u0) + u2 * 2^64: one multiply-add and one carry fold; at offset 2 they are
-// u0 * 2^64 + (u2:u1) * 2^96: one product and one subtraction; offset 1 takes the general 128-bit
-// reduction.  Multiplication by the radix-16 roots of unity (powers of w_16 = 2^12) thus costs
+// u0 * 2^64 + (u2:u1) * 2^96: one product and one subtraction; neg_mul_pow2 has offset 1.
+// Multiplication by the radix-16 roots of unity (powers of w_16 = 2^12) thus costs
 // three shifts and a short reduction instead of four wide products.
 template <int S>
 __device__ __forceinline__ uint64_t mul_pow2(uint64_t x)
 {
-    static_assert(S > 0 && S < 96, "shift out of range");
+    static_assert(S > 0 && S < 96 && S / 32 != 1 && S % 32, "shift out of range");
     constexpr int Q = S / 32, T = S % 32;
     const uint32_t x0 = lo32(x), x1 = hi32(x);
-    uint32_t u0, u1, u2;
-    if (T == 0) {
-        u0 = x0;
-        u1 = x1;
-        u2 = 0;
-    } else {
-        u0 = x0 << T;
-        u1 = __funnelshift_l(x0, x1, T);
-        u2 = x1 >> (32 - T);
-    }
+    const uint32_t u0 = x0 << T, u1 = __funnelshift_l(x0, x1, T), u2 = x1 >> (32 - T);
     if (Q == 0) {
         // (u1:u0) + u2 * 2^64 = (u1:u0) + u2 * (2^32 - 1): one carry at most, folded as 2^32 - 1
         uint32_t z0, z1, c;
@@ -234,7 +225,6 @@ __device__ __forceinline__ uint64_t mul_pow2(uint64_t x)
             : "r"(m));
         return mk64(z0, z1);
     }
-    if (Q == 1) return reduce128(0u, u0, u1, u2);
     // u0 * 2^64 + u1 * 2^96 + u2 * 2^128 = u0 * (2^32 - 1) - (u2 * 2^32 + u1), and u2 < 2^T <= 2^31
     // keeps the subtrahend below p
     uint64_t w;
@@ -242,45 +232,25 @@ __device__ __forceinline__ uint64_t mul_pow2(uint64_t x)
     return sub_c(w, mk64(u1, u2));
 }
 
-// Montgomery reduction: (r3:r2:r1:r0) * 2^-64 mod p, loose, of any 128-bit value hi * 2^64 + lo.  p = 1 - 2^32 + 2^64, so
+// Montgomery reduction (P. L. Montgomery, Modular multiplication without trial division, 1985) by 2^64:
+// (r3:r2:r1:r0) * 2^-64 mod p, loose, of a value hi * 2^64 + lo with hi at most 2^64 - 2^32.  p = 1 - 2^32 + 2^64, so
 // lo * p^-1 mod 2^64 is a = lo + (lo << 32), its product with p has the high half b = a - (a >> 32) - e (e the carry of
 // that sum), and the result is hi - b, plus p on a borrow (b < p, so one fold suffices).  With a1 = r1 + r0 that is
-// (hi + a1 + e) - (a1:r0): nine additions and no multiplication, where reduce128 takes eight and a product by 2^32 - 1.
-// SHORT leaves one out: the caller's hi is at most 2^64 - 2^32, so hi + a1 + e does not carry.
-template <bool SHORT>
+// (hi + a1 + e) - (a1:r0), whose first sum the bound on hi keeps in 64 bits: eight additions and no multiplication, where
+// reduce128 takes eight and a product by 2^32 - 1.
 __device__ __forceinline__ uint64_t mont_reduce(uint32_t r0, uint32_t r1, uint32_t r2, uint32_t r3)
 {
     uint32_t z0, z1, m;
-    if (SHORT)
-        asm("{\n\t.reg .u32 a;\n\t"
-            "add.cc.u32  a, %3, %4;\n\t"
-            "addc.cc.u32 %0, %5, a;\n\t"
-            "addc.u32    %1, %6, 0;\n\t"
-            "sub.cc.u32  %0, %0, %3;\n\t"
-            "subc.cc.u32 %1, %1, a;\n\t"
-            "subc.u32    %2, 0, 0;\n\t}"
-            : "=&r"(z0), "=&r"(z1), "=&r"(m)
-            : "r"(r0), "r"(r1), "r"(r2), "r"(r3));
-    else
-        asm("{\n\t.reg .u32 a, c;\n\t"
-            "add.cc.u32  a, %3, %4;\n\t"
-            "addc.cc.u32 %0, %5, a;\n\t"
-            "addc.cc.u32 %1, %6, 0;\n\t"
-            "addc.u32    c, 0, 0;\n\t"
-            "sub.cc.u32  %0, %0, %3;\n\t"
-            "subc.cc.u32 %1, %1, a;\n\t"
-            "subc.u32    %2, c, 0;\n\t}"
-            : "=&r"(z0), "=&r"(z1), "=&r"(m)
-            : "r"(r0), "r"(r1), "r"(r2), "r"(r3));
+    asm("{\n\t.reg .u32 a;\n\t"
+        "add.cc.u32  a, %3, %4;\n\t"
+        "addc.cc.u32 %0, %5, a;\n\t"
+        "addc.u32    %1, %6, 0;\n\t"
+        "sub.cc.u32  %0, %0, %3;\n\t"
+        "subc.cc.u32 %1, %1, a;\n\t"
+        "subc.u32    %2, 0, 0;\n\t}"
+        : "=&r"(z0), "=&r"(z1), "=&r"(m)
+        : "r"(r0), "r"(r1), "r"(r2), "r"(r3));
     return mk64(z0, z1) - (uint64_t)m;  // m = 2^32 - 1 on a borrow
-}
-
-// a * b * 2^-64, loose
-__device__ __forceinline__ uint64_t mont_mul(uint64_t a, uint64_t b)
-{
-    uint32_t r0, r1, r2, r3;
-    mul128(a, b, r0, r1, r2, r3);
-    return mont_reduce<false>(r0, r1, r2, r3);
 }
 
 // a * b * 2^-64 for b canonical (then the result is canonical: hi < p) or both at most MONT_MAX (then so is the result)
@@ -289,10 +259,10 @@ __device__ __forceinline__ uint64_t mont_mul_c(uint64_t a, uint64_t b)
 {
     uint32_t r0, r1, r2, r3;
     mul128(a, b, r0, r1, r2, r3);
-    return mont_reduce<true>(r0, r1, r2, r3);
+    return mont_reduce(r0, r1, r2, r3);
 }
 
-// -x * 2^S mod p for 32 <= S < 64, canonical: 2^96 = -1, so it is the Montgomery reduction of x << (S - 32), three
+// -x * 2^S mod p for 32 < S < 64, canonical: 2^96 = -1, so it is the Montgomery reduction of x << (S - 32), three
 // shifts and eight additions where the general reduction takes two products by 2^32 - 1 and a canonicalisation more.
 template <int S>
 __device__ __forceinline__ uint64_t neg_mul_pow2(uint64_t x)
@@ -300,7 +270,7 @@ __device__ __forceinline__ uint64_t neg_mul_pow2(uint64_t x)
     static_assert(S > 32 && S < 64, "shift out of range");
     constexpr int T = S - 32;
     const uint32_t x0 = lo32(x), x1 = hi32(x);
-    return mont_reduce<true>(x0 << T, __funnelshift_l(x0, x1, T), x1 >> (32 - T), 0);
+    return mont_reduce(x0 << T, __funnelshift_l(x0, x1, T), x1 >> (32 - T), 0);
 }
 
 // x^7 * 2^(-64 * 6) for x at most MONT_MAX
@@ -383,7 +353,7 @@ static inline uint64_t pow(uint64_t b, uint64_t e)
     }
     return acc;
 }
-// a times 2^64: the other factor of gl::mont_mul
+// a times 2^64: the other factor of gl::mont_mul_c
 static inline uint64_t mont(uint64_t a) { return mul(a, GL_EPS); }
 static inline uint64_t inv(uint64_t a) { return pow(a, GL_P - 2); }
 // W[k]: the reference's 2^k-th roots of unity (goldilocks_base_field.cpp:11-44), which are

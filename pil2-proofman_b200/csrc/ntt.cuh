@@ -32,7 +32,7 @@
 #define NTT_TWLG 26   // inter-window twiddles: powers of w_{2^26}; transforms up to 2^26 points
 #define NTT_TILE_MAX 8192
 
-// Every table holds its factors times 2^64 (Montgomery form), so a product with gl::mont_mul is the plain
+// Every table holds its factors times 2^64 (Montgomery form), so a product with gl::mont_mul_c is the plain
 // product of the element and the factor, and products of two factors stay in that form.
 __device__ uint64_t g_ntt_tw_lo_fwd[1 << 13];
 __device__ uint64_t g_ntt_tw_hi_fwd[1 << 13];
@@ -88,15 +88,12 @@ __device__ uint64_t g_ntt_w4096_inv[4096];  // w_4096^-i
 
 __device__ __forceinline__ uint32_t pad16(uint32_t i) { return i + (i >> 4); }
 
-// x * w_16^idx = x * 2^(12 idx) (idx constant once the butterfly loops are unrolled)
+// x * w_16^idx = x * 2^(12 idx) (idx constant once the butterfly loops are unrolled); idx 3 to 5 are gl::neg_mul_pow2
 __device__ __forceinline__ uint64_t mul_root16(uint64_t x, int idx)
 {
     switch (idx) {
     case 1: return gl::mul_pow2<12>(x);
     case 2: return gl::mul_pow2<24>(x);
-    case 3: return gl::mul_pow2<36>(x);
-    case 4: return gl::mul_pow2<48>(x);
-    case 5: return gl::mul_pow2<60>(x);
     case 6: return gl::mul_pow2<72>(x);
     case 7: return gl::mul_pow2<84>(x);
     default: return x;
