@@ -1,9 +1,8 @@
 """Cooperative Poseidon2 / Poseidon1 kernels (coop.cuh) at the boundaries where the tree builder
-switches between them and the one-thread-per-state kernels.
+switches between them and the tiled tensor core kernels.
 
-merkle::build_tree hashes the leaves cooperatively up to 8192 rows, builds levels of up to 8192
-parents cooperatively, and runs the last levels (<= 64 parents at W12/W16, <= 128 at W8) in one
-single-CTA launch.  Every case compares the whole tree buffer (leaves, padding, every level) with
+merkle::build_tree hashes the leaves cooperatively up to 4096 rows (8192 at arity 2) and builds levels of up
+to as many parents cooperatively, several levels a launch.  Every case compares the whole tree buffer (leaves, padding, every level) with
 the oracle's restatement of Poseidon2GoldilocksGPU::merkletree (poseidon2_goldilocks.cpp:129-175)
 or, for hash family 1, of PoseidonGoldilocks::merkletree (poseidon_goldilocks.cpp).
 Calls go through the C-ABI library; torch only allocates device memory.
@@ -36,14 +35,14 @@ def _tree(dev, m, arity):
     return d_tree.cpu().numpy().view(np.uint64)
 
 
-# (nrows, ncols, arity): leaf switch at 8192 rows; level switch at 8192 parents; tail limits
-# 64 parents (arity 3, 4) and 128 parents (arity 2); sponges of 1, 2 and 3 permutations
+# (nrows, ncols, arity): the switches of the leaves and of the levels, sponges of 1, 2 and 3 permutations
 CASES = [
-    (8192, 13, 4), (8193, 13, 4),          # cooperative / one-thread leaves, then cooperative levels
-    (32768, 3, 4), (32772, 3, 4),          # 8192 parents (cooperative) / 8193 (one-thread level)
-    (256, 25, 4), (257, 25, 4),            # straight into the tail / one cooperative level first
-    (192, 9, 3), (193, 9, 3), (8193, 8, 3),
-    (256, 5, 2), (257, 5, 2), (16386, 4, 2),
+    (4096, 13, 4), (4097, 13, 4),          # cooperative / tiled leaves, then cooperative levels
+    (16384, 3, 4), (16385, 3, 4),          # 4096 parents (cooperative) / 4097 (tiled level)
+    (4096, 20, 3), (4097, 20, 3), (12288, 3, 3), (12289, 3, 3),
+    (8192, 9, 2), (8193, 9, 2), (16384, 4, 2), (16385, 4, 2),
+    (8192, 13, 4), (8193, 13, 4), (32768, 3, 4), (32772, 3, 4), (8193, 8, 3), (16386, 4, 2),
+    (256, 25, 4), (257, 25, 4), (192, 9, 3), (193, 9, 3), (256, 5, 2), (257, 5, 2),
     (1, 7, 4), (2, 0, 4), (5, 30, 2),
 ]
 
@@ -66,7 +65,7 @@ def orc1():
 
 
 # Poseidon1: the same switch points (the oracle's Poseidon1 trees are slower, so fewer large ones)
-CASES1 = [(8192, 13, 4), (8193, 13, 4), (256, 25, 4), (257, 25, 4), (192, 9, 3), (193, 9, 3),
+CASES1 = [(4096, 13, 4), (4097, 13, 4), (16384, 3, 4), (16385, 3, 4), (8192, 4, 2), (8193, 4, 2), (8192, 13, 4), (8193, 13, 4), (256, 25, 4), (257, 25, 4), (192, 9, 3), (193, 9, 3),
           (256, 5, 2), (257, 5, 2), (1, 7, 4), (2, 0, 4), (5, 30, 2), (32772, 3, 4)]
 
 

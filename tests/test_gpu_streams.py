@@ -1,5 +1,6 @@
 """Commits beside other work on the device: a higher-priority stream gets in while a tree is hashed, and commits that
 run on several streams at once give the roots that they give one after another."""
+import threading
 import time
 
 import numpy as np
@@ -50,3 +51,48 @@ def test_higher_priority_work_enters_a_long_hash_launch(dev):
         low.synchronize()
         trees.append(a.elapsed_time(b))
     assert np.median(waits[1:]) < np.median(trees[1:]) / 3, (waits, trees)
+
+
+# log2 rows, log2 extended rows, columns, arity: cooperative and tiled sponges of every width, on an SM's whole tensor memory
+SHAPES = [(8, 9, 20, 4), (12, 13, 40, 4), (13, 14, 30, 2), (12, 13, 25, 3), (14, 15, 13, 4), (11, 14, 9, 2)]
+
+
+@pytest.mark.parametrize("family", [1, 2])
+def test_commits_on_several_streams(dev, family):
+    """Six commits at once, each on its stream and from its own host thread, several times over."""
+    pkg, torch = dev
+    pkg.set_native_hash_family(family)
+    work = []
+    for i, (nb, nbe, nc, ar) in enumerate(SHAPES):
+        trace = _empty(torch, nc << nb)
+        pkg.fill_random_device(trace, trace.numel(), 50 + i)
+        work.append((trace, _empty(torch, nc << nb), _empty(torch, nc << nbe), _empty(torch, pkg.tree_num_elements(1 << nbe, ar))))
+
+    def commit(i, stream, want_root):
+        nb, nbe, nc, ar = SHAPES[i]
+        trace, scratch, lde, tree = work[i]
+        return pkg.commit_device(lde, tree, trace, nb, nbe, nc, ar, scratch, stream=stream, want_root=want_root)
+
+    alone = [commit(i, None, True) for i in range(len(SHAPES))]
+    trees = [w[3].clone() for w in work]
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream() for _ in SHAPES]
+    roots = [None] * len(SHAPES)
+
+    def worker(i):
+        work[i][3].fill_(-1)
+        torch.cuda.current_stream().synchronize()
+        for _ in range(3):
+            commit(i, streams[i], False)
+        roots[i] = commit(i, streams[i], True)
+
+    threads = [threading.Thread(target=worker, args=(i,)) for i in range(len(SHAPES))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    torch.cuda.synchronize()
+    for i in range(len(SHAPES)):
+        assert (roots[i] == alone[i]).all(), SHAPES[i]
+        assert torch.equal(work[i][3], trees[i]), SHAPES[i]
+    assert pkg.load().b200_tma_wait_errors() == 0

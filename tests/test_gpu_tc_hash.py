@@ -57,6 +57,27 @@ def test_tree_at_the_tiles_edges(dev, arity, family, nrows):
         assert bad.size == 0, (nrows, ncols, arity, family, bad[:8])
 
 
+# Every sponge shape at every width and family, and three blocks with a ragged last one.
+@pytest.mark.parametrize("family", [1, 2])
+@pytest.mark.parametrize("arity", [2, 3, 4])
+@pytest.mark.parametrize("blocks,extra", COLS + [(3, 1), (4, -1)])
+def test_sponge_shapes(dev, arity, family, blocks, extra):
+    pkg, torch = dev
+    orc = oracle.Oracle(family=family)
+    pkg.set_native_hash_family(family)
+    nrows, ncols = 8320, blocks * (4 * arity - 4) + extra
+    m = oracle.random_field((nrows, ncols), ncols + 10 * arity + family)
+    if ncols:
+        m[0], m[-1] = np.uint64(2**64 - 1), np.uint64(oracle.P - 1)
+    exp = orc.merkletree(m % np.uint64(oracle.P), arity)
+    d_src = torch.from_numpy((m.reshape(-1) if m.size else np.zeros(1, np.uint64)).view(np.int64)).cuda()
+    tree = torch.zeros(exp.size, dtype=torch.int64, device="cuda")
+    pkg.merkletree_device(tree, d_src, ncols, 1, ncols, nrows, arity)
+    torch.cuda.synchronize()
+    bad = np.nonzero(tree.cpu().numpy().view(np.uint64) != exp)[0]
+    assert bad.size == 0, bad[:8]
+
+
 # One tile past a whole wave of CTAs that take a single tile a group (16 permutations a row and more), and past one of
 # CTAs that take two (8 permutations): the next wave's first CTA, with one group at work.
 @pytest.mark.parametrize("arity,nrows,blocks", [(4, 148 * 4 * 128 + 1, 17), (2, 148 * 8 * 128 + 1, 16),
