@@ -250,8 +250,9 @@ int b200_lde_rows_device(uint64_t *d_out, const uint64_t *d_lde, uint64_t NExt, 
 /* ---- Batched commit of many instances (device buffers) ---------------------------------
  * One plan covers a fixed set of instances (shapes and buffers).  A run performs, for all of
  * them together: one grouped transpose launch, one grouped launch per NTT window index, one
- * persistent leaf-sponge launch per arity (resident CTAs claim 128-row blocks of any instance
- * from a device counter), one grouped launch per tree level, one root gather.  With use_graph
+ * persistent leaf-sponge launch per arity (one CTA an SM, whose thread groups take 128-row blocks
+ * of any instance from a device counter), grouped launches of the tree levels (one of a large
+ * level, several small levels a launch), one root gather.  With use_graph
  * the first run captures that sequence into a CUDA graph and later runs replay it (stream
  * must then be a created stream).  Results are bit-identical to b200_commit_device per
  * instance.  The batched counterpart of the reference's per-instance commit loop

@@ -5,10 +5,11 @@
 // and every level of every tree is a separate launch.  Here one launch performs the same
 // phase for every instance of the batch:
 //   * grouped transpose, one launch per NTT window index (instances aligned on their last
-//     inverse window and on their first forward window), one launch per tree level index;
-//   * the leaf sponge is a persistent kernel: the four thread groups of one CTA per SM pull 128-row
-//     blocks of any instance from a device work counter until all rows are hashed, so
-//     instances of uneven size share the machine without tail effects;
+//     inverse window and on their first forward window), one launch per tree level while it is
+//     large, then several levels a launch;
+//   * the leaf sponge is a persistent kernel: the thread groups (four, eight at width 8) of one CTA per SM
+//     take 128-row blocks of any instance, widest first, from a device work counter until all rows are
+//     hashed, so instances of uneven size share the machine without tail effects;
 // and the whole sequence is captured once in a CUDA graph and replayed (BatchPlan).
 // Every kernel body is the plain path's body, so results are bit-identical to it.
 #pragma once

@@ -1,5 +1,5 @@
-// Cooperative Poseidon2 and Poseidon1 for work too small to fill the GPU with one thread per
-// state: the top levels of a tree and the leaves of tiny instances.
+// Cooperative Poseidon2 and Poseidon1 for work too small to fill the GPU with 128-row tiles
+// (tc_hash.cuh): the top levels of a tree and the leaves of tiny instances.
 //
 // One state per group of G lanes of a warp (G = 16 for W = 12 and 16, G = 8 for W = 8);
 // lane k of the group holds word k (lanes k >= W hold zero).  The S-boxes of a full round
@@ -7,9 +7,8 @@
 // row of M4 (small coefficients, two 64-bit sums of 32x32 products) and adds the column sum
 // over the blocks (xor shuffles over the block bits); the partial-round sum is an xor-shuffle
 // reduction over the group that runs beside x0's S-box.  A permutation then costs the latency
-// of about 30 S-box chains instead of 952 dependent multiplications: ~5x less time for a
-// state, at several times the instructions per state, so it is used only where the
-// one-thread-per-state kernels leave the GPU idle.  The arithmetic is the same modular
+// of about 30 S-box chains instead of 952 dependent multiplications (~8 us), at several times
+// the instructions per state, so it is used only where the tiled kernels leave the GPU idle.  The arithmetic is the same modular
 // arithmetic as poseidon2.cuh (loose words, 96-bit accumulators), so the canonical results are
 // identical.
 #pragma once
@@ -274,7 +273,7 @@ __device__ __forceinline__ uint64_t permute_fam(uint64_t x, int gbase, int k)
 // ---------------------------------------------------------------------------------
 constexpr int CTA_THREADS = 256;
 
-// Parent i of a tree level (semantics of merkle::node_one): the W = 4 * arity child words, zero
+// Parent i of a tree level (semantics of tch::node_tile): the W = 4 * arity child words, zero
 // past `pending`; the last parent writes the level's `pad` zero digests after its children.
 template <int W, int FAM>
 __device__ __forceinline__ void node_group(uint64_t *__restrict__ level, uint64_t pending, uint64_t pad,
@@ -349,7 +348,7 @@ inline int subtree_advance(uint64_t &pending, uint64_t &at)
     return levels;
 }
 
-// Row sponge of row `row` (semantics of merkle::leaf_row): the capacity starts at zero; each block
+// Row sponge of row `row` (semantics of tch::leaf_tile): the capacity starts at zero; each block
 // puts the next RATE columns (zero past the last) in lanes [0, RATE) and the previous output words
 // 0..3 in the capacity lanes; the digest is words 0..3.
 template <int W, int FAM = 2>

@@ -46,9 +46,9 @@ __device__ __forceinline__ void permute_fam(uint64_t *st)
         p2::permute_smem<W, TPB>(st);
 }
 
-// Row sponges of `nrows` rows, 128-row tiles over the groups of every CTA (tc_hash.cuh).  Against one thread a row with the state in shared memory and
-// every layer on the integer pipes, 2^20 rows (B200): Poseidon2 W16 x 256 columns 24.6 -> 16.4 ms (937 -> 1403 M
-// permutations/s), W12 x 128 13.9 -> 9.8, W8 x 64 9.6 -> 7.0; Poseidon1 W16 39.0 -> 16.4, W12 19.4 -> 9.7, W8 12.5 -> 7.0.
+// Row sponges of `nrows` rows, 128-row tiles over the groups of every CTA (tc_hash.cuh).  Against one thread a row with
+// the state in shared memory and every layer on the integer pipes, 2^20 rows (B200): Poseidon2 W16 x 256 columns 24.6 ->
+// 16.3 ms (937 -> 1413 M permutations/s), W12 x 128 13.9 -> 9.8, W8 x 64 9.6 -> 7.0; Poseidon1 W16 39.0 -> 16.4, W12 19.4 -> 9.7, W8 12.5 -> 7.0.
 template <int W, int FAM = 2>
 __global__ void __launch_bounds__(tch::Cfg<W>::THREADS, 1) leaf_hash_kernel(uint64_t *__restrict__ digests,
                                                                     const uint64_t *__restrict__ src, uint64_t rs,

@@ -655,10 +655,10 @@ extern "C" uint64_t gen_device_streams(void *d_buffers, uint64_t n_streams, uint
 // trace is large enough for the overlap to matter, a 16-column first block (nothing hides its
 // copy: the kernels start once it has landed; 128-byte row segments still copy at 47 GB/s), then
 // blocks of 24 and 48 columns, then 64-column blocks (512-byte row segments, which a 2-D copy
-// moves at the full 55 GB/s).  On an idle device the kernels of the blocks already landed (LDE
-// plus the chunked sponge, ~1.1 ms per 2^22-row column against ~0.6 ms of copy) must outlast the
-// next block's copy, or the GPU waits: after 16 columns that allows about 28 more, after 40
-// about 49 more.
+// moves at the full 55 GB/s).  On an idle device the kernels of the blocks already landed must
+// outlast the next block's copy, or the GPU waits.  The sizes are from kernels of ~1.1 ms per 2^22-row
+// column against ~0.6 ms of copy; at 0.75 ms now, blocks that grow more slowly were no faster (2^22 x 256
+// 241 against 237 ms, 2^20 x 256 60 against 58.5), because narrower row segments copy slower.
 static void commit_blocks(uint64_t nBits, uint64_t nCols, std::vector<uint64_t> &starts)
 {
     starts.assign(1, 0);

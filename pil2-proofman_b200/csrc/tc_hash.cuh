@@ -2,14 +2,14 @@
 //
 // The tables of tc_tables.h turn every linear layer (the external / MDS layers of the full rounds, and all
 // of the partial rounds but their S-boxes) into products of a state's bytes with a constant byte matrix.
-// One group of 256 threads owns 128 states: the states' bytes are the 128 rows of the left operand in shared
+// One group of 256 threads (128 at width 8) owns 128 states: the states' bytes are the 128 rows of the left operand in shared
 // memory (16-byte piece c of row r at c * 2048 + r * 16, so a thread's 16-byte accesses are conflict-free and
 // a state word is stored as it is), the accumulators are the 128 lanes of tensor memory, and a thread reads
 // its row's columns back and joins them to 64-bit words (join_word).
 //
-// What bounds it: the S-boxes' integer products (150 x^7 a width-16 permutation, at 0.85 clocks an SM each 128 of
-// the 207 clocks a permutation takes on a B200; IMAD.WIDE issues 25 lanes a clock and SM).  The tensor pipe is 12 %
-// busy, so no product is shaped for it: every layer goes through, also those with small coefficients, because
+// What bounds it: the S-boxes' integer products (150 x^7 a width-16 permutation, at 0.82 clocks an SM each in a loop of
+// nothing else 122 of the 206 clocks a permutation takes on a B200; IMAD.WIDE issues 25 lanes a clock and SM).  The
+// tensor pipe is 13 % busy, so no product is shaped for it: every layer goes through, also those with small coefficients, because
 // joining eight columns costs a third of the 128-bit sums that it replaces.  The S-boxes and joins run in
 // Montgomery form because that reduction needs no multiplication (gl64.cuh).
 //
