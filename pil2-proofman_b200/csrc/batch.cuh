@@ -206,7 +206,7 @@ __global__ void __launch_bounds__(tch::Cfg<W>::THREADS, 1) node_grouped(const No
     extern __shared__ __align__(128) uint8_t tc_sm[];
     __shared__ tch::Shared sh;
     tch::Group<W, FAM> G;
-    G.setup(tc_sm, sh);
+    G.setup(tc_sm, sh, split.groups);
     const tch::TileRange<W> r(split, G.id, total);
     for (uint64_t b = r.first; b < r.end; b += r.step) {
         const NodeEntry &E = e[find_entry(e, n, b)];
@@ -629,13 +629,13 @@ class Plan {
                                                          : tch::split<16>(L.blocks, 1, sms);
                 const NodeEntry *ne = (const NodeEntry *)ent;
                 if (family == 1) {
-                    if (L.width == 8) node_grouped<8, 1><<<split.ctas, tch::Cfg<8>::THREADS, tch::Smem<8>::BYTES, s>>>(ne, L.n, L.blocks, split);
-                    if (L.width == 12) node_grouped<12, 1><<<split.ctas, tch::Cfg<12>::THREADS, tch::Smem<12>::BYTES, s>>>(ne, L.n, L.blocks, split);
-                    if (L.width == 16) node_grouped<16, 1><<<split.ctas, tch::Cfg<16>::THREADS, tch::Smem<16>::BYTES, s>>>(ne, L.n, L.blocks, split);
+                    if (L.width == 8) node_grouped<8, 1><<<split.ctas, tch::Cfg<8>::GTHREADS * split.groups, tch::Smem<8>::bytes(split.groups), s>>>(ne, L.n, L.blocks, split);
+                    if (L.width == 12) node_grouped<12, 1><<<split.ctas, tch::Cfg<12>::GTHREADS * split.groups, tch::Smem<12>::bytes(split.groups), s>>>(ne, L.n, L.blocks, split);
+                    if (L.width == 16) node_grouped<16, 1><<<split.ctas, tch::Cfg<16>::GTHREADS * split.groups, tch::Smem<16>::bytes(split.groups), s>>>(ne, L.n, L.blocks, split);
                 } else {
-                    if (L.width == 8) node_grouped<8, 2><<<split.ctas, tch::Cfg<8>::THREADS, tch::Smem<8>::BYTES, s>>>(ne, L.n, L.blocks, split);
-                    if (L.width == 12) node_grouped<12, 2><<<split.ctas, tch::Cfg<12>::THREADS, tch::Smem<12>::BYTES, s>>>(ne, L.n, L.blocks, split);
-                    if (L.width == 16) node_grouped<16, 2><<<split.ctas, tch::Cfg<16>::THREADS, tch::Smem<16>::BYTES, s>>>(ne, L.n, L.blocks, split);
+                    if (L.width == 8) node_grouped<8, 2><<<split.ctas, tch::Cfg<8>::GTHREADS * split.groups, tch::Smem<8>::bytes(split.groups), s>>>(ne, L.n, L.blocks, split);
+                    if (L.width == 12) node_grouped<12, 2><<<split.ctas, tch::Cfg<12>::GTHREADS * split.groups, tch::Smem<12>::bytes(split.groups), s>>>(ne, L.n, L.blocks, split);
+                    if (L.width == 16) node_grouped<16, 2><<<split.ctas, tch::Cfg<16>::GTHREADS * split.groups, tch::Smem<16>::bytes(split.groups), s>>>(ne, L.n, L.blocks, split);
                 }
                 break;
             }

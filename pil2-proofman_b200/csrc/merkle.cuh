@@ -58,7 +58,7 @@ __global__ void __launch_bounds__(tch::Cfg<W>::THREADS, 1) leaf_hash_kernel(uint
     extern __shared__ __align__(128) uint8_t tc_sm[];
     __shared__ tch::Shared sh;
     tch::Group<W, FAM> G;
-    G.setup(tc_sm, sh);
+    G.setup(tc_sm, sh, split.groups);
     const tch::TileRange<W> r(split, G.id, (nrows + 127) / 128);
     for (uint64_t t = r.first; t < r.end; t += r.step) {
         tch::leaf_tile(G, digests, src, rs, cs, ncols, nrows, t, resume != 0);
@@ -76,7 +76,7 @@ __global__ void __launch_bounds__(tch::Cfg<W>::THREADS, 1) node_kernel(uint64_t 
     extern __shared__ __align__(128) uint8_t tc_sm[];
     __shared__ tch::Shared sh;
     tch::Group<W, FAM> G;
-    G.setup(tc_sm, sh);
+    G.setup(tc_sm, sh, split.groups);
     const tch::TileRange<W> r(split, G.id, (parents + 127) / 128);
     for (uint64_t t = r.first; t < r.end; t += r.step) {
         tch::node_tile(G, level, pending, pad, parents, out, t);
@@ -146,7 +146,7 @@ cudaError_t build_levels(uint64_t *d_tree, uint64_t nrows, cudaStream_t stream)
             continue;
         }
         const tch::Split split = tch::split<W>((parents + 127) / 128, 1);
-        node_kernel<W, FAM><<<split.ctas, tch::Cfg<W>::THREADS, tch::Smem<W>::BYTES, stream>>>(
+        node_kernel<W, FAM><<<split.ctas, tch::Cfg<W>::GTHREADS * split.groups, tch::Smem<W>::bytes(split.groups), stream>>>(
             lvl, pending, pad, parents, lvl + (pending + pad) * 4, split);
         prof::count();
         base += (pending + pad) * 4;
@@ -161,7 +161,7 @@ cudaError_t hash_rows(uint64_t *digests, const uint64_t *src, uint64_t rs, uint6
                       bool resume, cudaStream_t stream)
 {
     const tch::Split split = tch::split<W>((nrows + 127) / 128, (ncols + W - 5) / (W - 4));
-    leaf_hash_kernel<W, FAM><<<split.ctas, tch::Cfg<W>::THREADS, tch::Smem<W>::BYTES, stream>>>(
+    leaf_hash_kernel<W, FAM><<<split.ctas, tch::Cfg<W>::GTHREADS * split.groups, tch::Smem<W>::bytes(split.groups), stream>>>(
         digests, src, rs, cs, ncols, nrows, resume ? 1 : 0, split);
     prof::count();
     return cudaGetLastError();

@@ -45,7 +45,8 @@ constexpr uint32_t WAIT_LIMIT = 1u << 20;  // try_wait rounds before a thread gi
 template <int W>
 struct Smem {
     static constexpr int GROUP = (Shape<W>::CHX + YCH) * 2048;  // state rows and a block's y rows
-    static constexpr int BYTES = Shape<W>::BYTES + Cfg<W>::GROUPS * GROUP;
+    static constexpr int bytes(int groups) { return Shape<W>::BYTES + groups * GROUP; }
+    static constexpr int BYTES = bytes(Cfg<W>::GROUPS);
 };
 
 __device__ __forceinline__ uint32_t smem_addr(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -173,7 +174,7 @@ __device__ __forceinline__ void store_words(uint64_t *p, const uint64_t (&v)[N])
 // A CTA's barriers and tensor memory address.
 struct Shared {
     uint64_t mbar[MAX_GROUPS];
-    uint32_t tmem;
+    uint32_t tmem, columns;
 };
 
 // A thread's view of its group.
@@ -200,20 +201,27 @@ struct Group {
         sts128(row + (uint32_t)(i >> 1) * 2048, x, y);
     }
 
-    // Tables into shared memory, tensor memory, barriers.  All threads of the CTA.
-    __device__ __forceinline__ void setup(uint8_t *sm, Shared &sh)
+    // Tables into shared memory, tensor memory, barriers.  All threads of the CTA, which has `groups` groups.
+    __device__ __forceinline__ void setup(uint8_t *sm, Shared &sh, uint32_t groups = GROUPS)
     {
         const uint32_t warp = threadIdx.x >> 5;
-        const uint4 *src = reinterpret_cast<const uint4 *>(g_tc_tab[FAM - 1][W / 4 - 2]);
-        for (uint32_t i = threadIdx.x; i < (uint32_t)Shape<W>::BYTES / 16; i += THREADS)
-            reinterpret_cast<uint4 *>(sm)[i] = __ldg(src + i);
+        const uint8_t *src = g_tc_tab[FAM - 1][W / 4 - 2];
+        tab = smem_addr(sm);
+        // asynchronous copies: with one group a CTA, loads through registers took 3 us longer
+        for (uint32_t i = threadIdx.x * 16; i < (uint32_t)Shape<W>::BYTES; i += groups * GTHREADS * 16)
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(tab + i), "l"(__cvta_generic_to_global(src + i)) : "memory");
+        asm volatile("cp.async.commit_group;" ::: "memory");
         if (warp == 0) {
-            asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_addr(&sh.tmem))
+            const uint32_t columns = groups * Cfg<W>::COLS;  // a power of two wherever groups < GROUPS (split)
+            if (threadIdx.x == 0) sh.columns = groups == GROUPS ? 512 : columns;
+            asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(&sh.tmem)),
+                         "r"(groups == GROUPS ? 512 : columns)
                          : "memory");
             asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
         }
         if (threadIdx.x < GROUPS)
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(sh.mbar + threadIdx.x)) : "memory");
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -222,7 +230,6 @@ struct Group {
         id = threadIdx.x / GTHREADS;
         half = (threadIdx.x >> 7) % SPLIT;
         const uint32_t r = threadIdx.x & 127;
-        tab = smem_addr(sm);
         row = tab + Shape<W>::BYTES + id * Smem<W>::GROUP + r * 16;
         tmem = sh.tmem + id * Cfg<W>::COLS + ((warp & 3) << 21);
         mbar = smem_addr(sh.mbar + id);
@@ -308,7 +315,7 @@ struct Group {
         __syncthreads();
         if (threadIdx.x < 32) {
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(sh.tmem));
+            asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(sh.tmem), "r"(sh.columns));
         }
     }
 
@@ -395,10 +402,10 @@ struct Group {
     }
 };
 
-// Tiles of a launch over its CTAs: waves of `lanes` CTAs, `rounds` tiles a group and wave; a wave's first tiles go
-// to different CTAs, so that few tiles spread over the SMs.
+// Tiles of a launch over its CTAs of `groups` groups: waves of `lanes` CTAs, `rounds` tiles a group and wave; a wave's
+// first tiles go to different CTAs, so that few tiles spread over the SMs.
 struct Split {
-    uint32_t lanes, rounds, ctas;
+    uint32_t lanes, rounds, ctas, groups;
 };
 
 // A group's tiles: for (t = first; t < end; t += step).
@@ -407,7 +414,7 @@ struct TileRange {
     uint64_t first, end, step;
     __device__ __forceinline__ TileRange(const Split &s, uint32_t group, uint64_t tiles)
     {
-        step = (uint64_t)s.lanes * Cfg<W>::GROUPS;
+        step = (uint64_t)s.lanes * s.groups;
         const uint64_t wave = step * s.rounds, begin = blockIdx.x / s.lanes * wave;
         first = begin + (uint64_t)group * s.lanes + blockIdx.x % s.lanes;
         end = tiles - begin < wave ? tiles : begin + wave;
@@ -539,14 +546,20 @@ inline cudaError_t init_tables()
 // at high priority 1 ms into a tree of 2^20 x 256 waited 14.9 ms (whole sponge 16.4), with these 0.08; the trees take the
 // same (16.60 and 16.61 ms; 2^20 x 24: 1.86 both).  Half as many permutations a CTA take 2 % more at 24 columns: a table
 // load and tensor memory setup are a few microseconds each.
+// At width 8 a launch of one or two tiles an SM has CTAs of as many groups (64 or 84 KB of shared memory, 64 or 128 tensor
+// memory columns), so three or two launches of different streams share an SM; with CTAs of eight groups they queued with
+// one or two at work.  48 commits of 2^13 x 40 at arity 2 on 16 streams: 10.1 -> 6.1 ms (7.7 with the one-thread-a-row
+// kernels), on one stream 17.2 -> 17.0.  At width 16 the tables alone keep a second CTA out (2 x 134 KB), and there and at
+// width 12 the same commits took 0.88-0.99 of those kernels' time as they are.
 constexpr uint64_t CTA_PERMS = 16;
 template <int W>
 inline Split split(uint64_t tiles, uint64_t perms, uint64_t sms)
 {
     const uint64_t rounds = perms >= CTA_PERMS ? 1 : perms ? CTA_PERMS / perms : CTA_PERMS;
-    const uint64_t lanes = tiles < sms ? tiles : sms, wave = rounds * Cfg<W>::GROUPS * lanes;
+    const uint32_t groups = W != 8 ? Cfg<W>::GROUPS : tiles <= sms ? 1 : tiles <= 2 * sms ? 2 : Cfg<W>::GROUPS;
+    const uint64_t lanes = tiles < sms ? tiles : sms, wave = rounds * groups * lanes;
     const uint64_t rest = tiles % wave;
-    return Split{(uint32_t)lanes, (uint32_t)rounds, (uint32_t)(tiles / wave * lanes + (rest < lanes ? rest : lanes))};
+    return Split{(uint32_t)lanes, (uint32_t)rounds, (uint32_t)(tiles / wave * lanes + (rest < lanes ? rest : lanes)), groups};
 }
 
 // the same on the current device

@@ -96,3 +96,38 @@ def test_commits_on_several_streams(dev, family):
         assert (roots[i] == alone[i]).all(), SHAPES[i]
         assert torch.equal(work[i][3], trees[i]), SHAPES[i]
     assert pkg.load().b200_tma_wait_errors() == 0
+
+
+def test_small_launches_share_the_sms(dev):
+    """Eight streams of arity-2 commits whose sponges are 128 tiles each: CTAs of one group share an SM, so they take
+    0.42 of the time of the same commits on one stream; while a CTA of eight groups took the SM for one tile, 0.72."""
+    pkg, torch = dev
+    pkg.set_native_hash_family(2)
+    nb, nbe, nc, ar, n = 13, 14, 100, 2, 8
+    work = [(_empty(torch, nc << nb), _empty(torch, nc << nb), _empty(torch, nc << nbe),
+             _empty(torch, pkg.tree_num_elements(1 << nbe, ar))) for _ in range(n)]
+    for i, w in enumerate(work):
+        pkg.fill_random_device(w[0], w[0].numel(), i)
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream() for _ in range(n)]
+    main = torch.cuda.current_stream()
+
+    def run(over):
+        ms = []
+        for _ in range(6):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            for s in over:
+                s.wait_event(a)
+            for k in range(3 * n):
+                trace, scratch, lde, tree = work[k % n]
+                pkg.commit_device(lde, tree, trace, nb, nbe, nc, ar, scratch, stream=over[k % n % len(over)], want_root=False)
+            for s in over:
+                main.wait_stream(s)
+            b.record()
+            torch.cuda.synchronize()
+            ms.append(a.elapsed_time(b))
+        return min(ms[1:])
+
+    together, apart = run(streams), run(streams[:1])
+    assert together < 0.57 * apart, (together, apart)
