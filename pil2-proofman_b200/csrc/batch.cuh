@@ -173,14 +173,14 @@ inline cudaError_t set_grouped_fixed_attrs()
 // instances of 2^10-2^17 rows the same.
 template <int W, int FAM>
 __global__ void __launch_bounds__(tch::Cfg<W>::THREADS, 1)
-    leaf_persistent(const LeafEntry *e, int n, uint64_t total, unsigned long long *counter)
+    leaf_persistent(const LeafEntry *e, int n, uint64_t total, unsigned long long *counter, uint32_t groups)
 {
     extern __shared__ __align__(128) uint8_t tc_sm[];
     __shared__ tch::Shared sh;
     __shared__ uint64_t claim[tch::Cfg<W>::GROUPS];
     __shared__ LeafEntry entry[tch::Cfg<W>::GROUPS];  // the claimed block's instance, staged for the group
     tch::Group<W, FAM> G;
-    G.setup(tc_sm, sh);
+    G.setup(tc_sm, sh, groups);
     uint64_t next = blockIdx.x + (uint64_t)gridDim.x * G.id;
     for (;;) {
         if (G.issuer) {
@@ -193,7 +193,7 @@ __global__ void __launch_bounds__(tch::Cfg<W>::THREADS, 1)
         if (b >= total) break;
         const LeafEntry &L = entry[G.id];
         tch::leaf_tile(G, L.digests, L.src, 1, L.nrows, L.ncols, L.nrows, b - L.begin, false);
-        if (G.issuer) next = (uint64_t)gridDim.x * tch::Cfg<W>::GROUPS + atomicAdd(counter, 1ull);
+        if (G.issuer) next = (uint64_t)gridDim.x * groups + atomicAdd(counter, 1ull);
         if (G.gave_up()) break;
     }
     G.finish(sh);
@@ -598,14 +598,18 @@ class Plan {
             case 2: {
                 const unsigned ctas = (unsigned)std::min<uint64_t>(L.blocks, (uint64_t)leaf_ctas);
                 const LeafEntry *le = (const LeafEntry *)ent;
+                const uint64_t sms = (uint64_t)leaf_ctas;
+                const uint32_t groups = L.width == 8    ? tch::few_groups<8>(L.blocks, sms)
+                                        : L.width == 12 ? tch::few_groups<12>(L.blocks, sms)
+                                                        : tch::few_groups<16>(L.blocks, sms);
                 if (family == 1) {
-                    if (L.width == 8) leaf_persistent<8, 1><<<ctas, tch::Cfg<8>::THREADS, tch::Smem<8>::BYTES, s>>>(le, L.n, L.blocks, ctr + L.smem);
-                    if (L.width == 12) leaf_persistent<12, 1><<<ctas, tch::Cfg<12>::THREADS, tch::Smem<12>::BYTES, s>>>(le, L.n, L.blocks, ctr + L.smem);
-                    if (L.width == 16) leaf_persistent<16, 1><<<ctas, tch::Cfg<16>::THREADS, tch::Smem<16>::BYTES, s>>>(le, L.n, L.blocks, ctr + L.smem);
+                    if (L.width == 8) leaf_persistent<8, 1><<<ctas, tch::Cfg<8>::GTHREADS * groups, tch::Smem<8>::bytes(groups), s>>>(le, L.n, L.blocks, ctr + L.smem, groups);
+                    if (L.width == 12) leaf_persistent<12, 1><<<ctas, tch::Cfg<12>::GTHREADS * groups, tch::Smem<12>::bytes(groups), s>>>(le, L.n, L.blocks, ctr + L.smem, groups);
+                    if (L.width == 16) leaf_persistent<16, 1><<<ctas, tch::Cfg<16>::GTHREADS * groups, tch::Smem<16>::bytes(groups), s>>>(le, L.n, L.blocks, ctr + L.smem, groups);
                 } else {
-                    if (L.width == 8) leaf_persistent<8, 2><<<ctas, tch::Cfg<8>::THREADS, tch::Smem<8>::BYTES, s>>>(le, L.n, L.blocks, ctr + L.smem);
-                    if (L.width == 12) leaf_persistent<12, 2><<<ctas, tch::Cfg<12>::THREADS, tch::Smem<12>::BYTES, s>>>(le, L.n, L.blocks, ctr + L.smem);
-                    if (L.width == 16) leaf_persistent<16, 2><<<ctas, tch::Cfg<16>::THREADS, tch::Smem<16>::BYTES, s>>>(le, L.n, L.blocks, ctr + L.smem);
+                    if (L.width == 8) leaf_persistent<8, 2><<<ctas, tch::Cfg<8>::GTHREADS * groups, tch::Smem<8>::bytes(groups), s>>>(le, L.n, L.blocks, ctr + L.smem, groups);
+                    if (L.width == 12) leaf_persistent<12, 2><<<ctas, tch::Cfg<12>::GTHREADS * groups, tch::Smem<12>::bytes(groups), s>>>(le, L.n, L.blocks, ctr + L.smem, groups);
+                    if (L.width == 16) leaf_persistent<16, 2><<<ctas, tch::Cfg<16>::GTHREADS * groups, tch::Smem<16>::bytes(groups), s>>>(le, L.n, L.blocks, ctr + L.smem, groups);
                 }
                 break;
             }

@@ -38,6 +38,12 @@ struct Cfg {
     static constexpr int GROUPS = W == 8 ? 8 : 4, SPLIT = W == 8 ? 1 : 2;
     static constexpr int GTHREADS = 128 * SPLIT, THREADS = GTHREADS * GROUPS, COLS = 8 * W;
     static_assert(GROUPS * COLS <= 512 && GROUPS <= 15, "tensor memory columns, barriers");
+    // an allocation is a power of two
+    static __device__ __forceinline__ uint32_t columns(uint32_t groups)
+    {
+        const uint32_t n = groups * COLS;
+        return n > 256 ? 512 : n > 128 ? 256 : n > 64 ? 128 : 64;
+    }
 };
 constexpr int MAX_GROUPS = 8;
 constexpr uint32_t WAIT_LIMIT = 1u << 20;  // try_wait rounds before a thread gives up
@@ -212,10 +218,10 @@ struct Group {
             asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(tab + i), "l"(__cvta_generic_to_global(src + i)) : "memory");
         asm volatile("cp.async.commit_group;" ::: "memory");
         if (warp == 0) {
-            const uint32_t columns = groups * Cfg<W>::COLS;  // a power of two wherever groups < GROUPS (split)
-            if (threadIdx.x == 0) sh.columns = groups == GROUPS ? 512 : columns;
+            const uint32_t columns = Cfg<W>::columns(groups);
+            if (threadIdx.x == 0) sh.columns = columns;
             asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(&sh.tmem)),
-                         "r"(groups == GROUPS ? 512 : columns)
+                         "r"(columns)
                          : "memory");
             asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
         }
@@ -540,23 +546,31 @@ inline cudaError_t init_tables()
     return upload<16>();
 }
 
+// Groups of a CTA of a launch over `tiles` tiles.  Up to one tile an SM (two at width 8) as many as it has, so that launches
+// of different streams share an SM where tables, rows and tensor memory columns fit more than once: three CTAs of 64 KB and
+// 64 columns at width 8 (two of 84 KB with two groups), two of 96 KB and 128 columns at width 12.  With all groups they
+// queued, one of eight or four at work: 48 commits of 2^13 x 40 on 16 streams 10.1 -> 6.1 ms at arity 2 (7.7 with the
+// one-thread-a-row kernels) and 6.0 -> 4.4 at arity 3 (6.3), on one stream 17.2 -> 17.0 and 12.3 -> 12.2.  At width 16 the
+// tables keep a second CTA out (2 x 134 KB).
+template <int W>
+inline uint32_t few_groups(uint64_t tiles, uint64_t sms)
+{
+    if (W < 16 && tiles <= sms) return 1;
+    return W == 8 && tiles <= 2 * sms ? 2 : Cfg<W>::GROUPS;
+}
+
 // Launch over `tiles` 128-row tiles of `perms` permutations a row.  A CTA holds its SM to its end, and a kernel of a
 // higher-priority stream enters at CTA ends only, so a group takes the tiles of 16 permutations (0.9-1.0 ms with every
 // group at work) or one wider tile, and the next CTA goes on.  With one CTA an SM for all tiles, query openings issued
 // at high priority 1 ms into a tree of 2^20 x 256 waited 14.9 ms (whole sponge 16.4), with these 0.08; the trees take the
 // same (16.60 and 16.61 ms; 2^20 x 24: 1.86 both).  Half as many permutations a CTA take 2 % more at 24 columns: a table
 // load and tensor memory setup are a few microseconds each.
-// At width 8 a launch of one or two tiles an SM has CTAs of as many groups (64 or 84 KB of shared memory, 64 or 128 tensor
-// memory columns), so three or two launches of different streams share an SM; with CTAs of eight groups they queued with
-// one or two at work.  48 commits of 2^13 x 40 at arity 2 on 16 streams: 10.1 -> 6.1 ms (7.7 with the one-thread-a-row
-// kernels), on one stream 17.2 -> 17.0.  At width 16 the tables alone keep a second CTA out (2 x 134 KB), and there and at
-// width 12 the same commits took 0.88-0.99 of those kernels' time as they are.
 constexpr uint64_t CTA_PERMS = 16;
 template <int W>
 inline Split split(uint64_t tiles, uint64_t perms, uint64_t sms)
 {
     const uint64_t rounds = perms >= CTA_PERMS ? 1 : perms ? CTA_PERMS / perms : CTA_PERMS;
-    const uint32_t groups = W != 8 ? Cfg<W>::GROUPS : tiles <= sms ? 1 : tiles <= 2 * sms ? 2 : Cfg<W>::GROUPS;
+    const uint32_t groups = few_groups<W>(tiles, sms);
     const uint64_t lanes = tiles < sms ? tiles : sms, wave = rounds * groups * lanes;
     const uint64_t rest = tiles % wave;
     return Split{(uint32_t)lanes, (uint32_t)rounds, (uint32_t)(tiles / wave * lanes + (rest < lanes ? rest : lanes)), groups};

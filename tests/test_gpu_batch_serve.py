@@ -136,9 +136,9 @@ def test_one_shot_batch_entry(pkg, torch_cuda):
 
 
 # The batched leaf sponge gives every group its first 128-row block by its place and the others from a counter: blocks
-# for one group, for fewer groups than the 148 CTAs have (4 each, 8 at arity 2), and some past them.
+# for one group, for fewer groups than the 148 CTAs have (4 each, 8 at arity 2; 1 or 2 of a small batch), and some past them.
 @pytest.mark.parametrize("arity,family,count,nbits", [(4, 2, 1, 6), (4, 2, 3, 10), (4, 2, 5, 13), (4, 1, 5, 13), (3, 2, 5, 13),
-                                                      (2, 2, 3, 11), (2, 2, 10, 13)])
+                                                      (3, 2, 1, 13), (2, 2, 3, 11), (2, 2, 3, 12), (2, 2, 10, 13)])
 def test_batch_leaf_blocks(pkg, torch_cuda, arity, family, count, nbits):
     torch = torch_cuda
     pkg.init(0)

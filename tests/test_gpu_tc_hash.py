@@ -78,6 +78,25 @@ def test_sponge_shapes(dev, arity, family, blocks, extra):
     assert bad.size == 0, bad[:8]
 
 
+# CTAs of one group up to a tile an SM at widths 8 and 12, of two up to two tiles at width 8: the last rows of each and the next.
+@pytest.mark.parametrize("family", [1, 2])
+@pytest.mark.parametrize("arity,nrows", [(2, 148 * 128), (2, 148 * 128 + 1), (2, 2 * 148 * 128), (2, 2 * 148 * 128 + 1),
+                                         (3, 148 * 128), (3, 148 * 128 + 1)])
+def test_tree_at_the_group_rule(dev, arity, nrows, family):
+    pkg, torch = dev
+    orc = oracle.Oracle(family=family)
+    pkg.set_native_hash_family(family)
+    ncols = 4 * arity - 3
+    m = oracle.random_field((nrows, ncols), nrows + family)
+    exp = orc.merkletree(m, arity)
+    d_src = torch.from_numpy(np.ascontiguousarray(m.T).view(np.int64)).cuda()
+    tree = torch.zeros(exp.size, dtype=torch.int64, device="cuda")
+    pkg.merkletree_device(tree, d_src, 1, nrows, ncols, nrows, arity)
+    torch.cuda.synchronize()
+    bad = np.nonzero(tree.cpu().numpy().view(np.uint64) != exp)[0]
+    assert bad.size == 0, bad[:8]
+
+
 # One tile past a whole wave of CTAs that take a single tile a group (16 permutations a row and more), and past one of
 # CTAs that take two (8 permutations): the next wave's first CTA, with one group at work.
 @pytest.mark.parametrize("arity,nrows,blocks", [(4, 148 * 4 * 128 + 1, 17), (2, 148 * 8 * 128 + 1, 16),
