@@ -13,8 +13,8 @@
 // joining eight columns costs a third of the 128-bit sums that it replaces.  The S-boxes and joins run in
 // Montgomery form because that reduction needs no multiplication (gl64.cuh).
 //
-// At width 12 and 16 a CTA is four groups, one CTA an SM: the tables take 106 KB of shared memory at width 16, each
-// group 28 KB and a quarter of the tensor memory (128 columns, a whole layer's).  Two threads share a row (each takes
+// At width 12 and 16 a CTA is four groups, one CTA an SM (fewer groups where a launch has few tiles, few_groups): the
+// tables take 106 KB of shared memory at width 16, each group 28 KB and a quarter of the tensor memory (128 columns, a whole layer's).  Two threads share a row (each takes
 // half its words, and every other run of partial rounds), so 32 warps hide the barriers and latencies: 1000 rows of
 // 40 columns take 16 % less than with one thread a row, large launches the same.  At width 8 a layer has 64
 // columns and the tables take 44 KB, so eight groups fit with one thread a row: 2^20 rows x 64 columns 7.5 -> 7.0 ms.
