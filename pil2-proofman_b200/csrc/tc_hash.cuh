@@ -14,8 +14,8 @@
 // Montgomery form because that reduction needs no multiplication (gl64.cuh).
 //
 // At width 12 and 16 a CTA is four groups, one CTA an SM (fewer groups where a launch has few tiles, few_groups): the
-// tables take 106 KB of shared memory at width 16, each group 28 KB and a quarter of the tensor memory (128 columns, a whole layer's).  Two threads share a row (each takes
-// half its words, and every other run of partial rounds), so 32 warps hide the barriers and latencies: 1000 rows of
+// tables take 106 KB of shared memory at width 16, each group 28 KB and a quarter of the tensor memory (128 columns, a
+// whole layer's).  Two threads share a row (each takes half its words, and every other run of partial rounds), so 32 warps hide the barriers and latencies: 1000 rows of
 // 40 columns take 16 % less than with one thread a row, large launches the same.  At width 8 a layer has 64
 // columns and the tables take 44 KB, so eight groups fit with one thread a row: 2^20 rows x 64 columns 7.5 -> 7.0 ms.
 // Groups run independently, so one's products and barriers run under the others' S-boxes.
@@ -563,7 +563,8 @@ inline uint32_t few_groups(uint64_t tiles, uint64_t sms)
 // higher-priority stream enters at CTA ends only, so a group takes the tiles of 16 permutations (0.9-1.0 ms with every
 // group at work) or one wider tile, and the next CTA goes on.  With one CTA an SM for all tiles, query openings issued
 // at high priority 1 ms into a tree of 2^20 x 256 waited 14.9 ms (whole sponge 16.4), with these 0.08; the trees take the
-// same (16.60 and 16.61 ms; 2^20 x 24: 1.86 both).  Half as many permutations a CTA take 2 % more at 24 columns: a table
+// same (16.60 and 16.61 ms; 2^20 x 24: 1.86 both); at most 1 % more where a second wave is short of tiles (a commit of
+// 2^16 x 126 at arity 3: 1.86 -> 1.88).  Half as many permutations a CTA take 2 % more at 24 columns: a table
 // load and tensor memory setup are a few microseconds each.
 constexpr uint64_t CTA_PERMS = 16;
 template <int W>
